@@ -58,16 +58,20 @@ int pipe_init(cupcfd_gpu_mesh *m) {
     return CUPCFD_E_SUCCESS;
 }
 
-inline SellView sell(const cupcfd_gpu_mesh *m) { return SellView{m->sell.slicePtr, m->sell.inc, m->sell.width}; }
+inline SellView sell(const cupcfd_gpu_mesh *m) {
+    return SellView{m->sell.slicePtr, m->sell.inc, m->sell.width, m->sell.runHead, m->sell.runs};
+}
 
-// The width the L2-prefetch kernels are specialised for (kernels_pf.cuh:
-// WF), set by tiles_setup: 6 when every cell has exactly six incidences
-// (all hexahedral meshes), else 0 (the general kernels).
-inline int full_width(const cupcfd_gpu_mesh *m) { return m->fullWidth; }
-// launches the L2-prefetch kernel template K at the mesh's full width
+// The list form the L2-prefetch kernels are specialised for (kernels_pf.cuh:
+// WF): 6 when every cell has exactly six incidences (all hexahedral meshes),
+// -6 when those lists also have their run form (struct Sell), else 0 (the
+// general kernels).
+inline int list_form(const cupcfd_gpu_mesh *m) { return m->fullWidth == 6 && m->sell.runs ? -6 : m->fullWidth; }
+// launches the L2-prefetch kernel template K for the mesh's list form
 #define CG_LAUNCH_PF_BLOCK(m, K, grid, block, st, ...)                          \
     do {                                                                        \
-        if (full_width(m) == 6) K<6><<<(grid), (block), 0, (st)>>>(__VA_ARGS__); \
+        if (list_form(m) == -6) K<-6><<<(grid), (block), 0, (st)>>>(__VA_ARGS__); \
+        else if (list_form(m) == 6) K<6><<<(grid), (block), 0, (st)>>>(__VA_ARGS__); \
         else K<0><<<(grid), (block), 0, (st)>>>(__VA_ARGS__);                   \
     } while (0)
 #define CG_LAUNCH_PF(m, K, grid, st, ...) CG_LAUNCH_PF_BLOCK(m, K, grid, BLK, st, __VA_ARGS__)
@@ -150,21 +154,31 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
     const char *fw = std::getenv("CUPCFD_FULL_WIDTH");
     m->fullWidth = m->sell.width == 6 && (int64_t) m->nInc == 6 * (int64_t) m->nC &&
                    !(fw && std::strcmp(fw, "0") == 0) ? 6 : 0;
-    const bool w6 = full_width(m) == 6;
+    const int wf = list_form(m);
+    if (wf == -6) {
+        TileDesc *dr;
+        CG_TRY(m->alloc(&dr, (size_t) m->nTiles));
+        k_tile_desc_runs<<<grid_for(m->nTiles, BLK), BLK, 0, st>>>(m->nTiles, m->sell.nSlices, m->sell.nRuns,
+                                                                  m->sell.runHead, desc, dr);
+        CG_LAUNCHED();
+        m->tileDescRuns = dr;
+    }
+#define PF_KERNEL(K) (wf == -6 ? (const void *) K<-6> : wf == 6 ? (const void *) K<6> : (const void *) K<0>)
     const void *pfKern[] = {
-        w6 ? (const void *) k_fwd_f32_pf<6> : (const void *) k_fwd_f32_pf<0>,
-        w6 ? (const void *) k_adj_f32_pf<6> : (const void *) k_adj_f32_pf<0>,
-        w6 ? (const void *) k_fwd_f64_pf<6> : (const void *) k_fwd_f64_pf<0>,
-        w6 ? (const void *) k_adj_f64_pf<6> : (const void *) k_adj_f64_pf<0>,
-        w6 ? (const void *) k_fwd_madj_f32_pf<6> : (const void *) k_fwd_madj_f32_pf<0>,
-        w6 ? (const void *) k_gadj_f32_pf<6> : (const void *) k_gadj_f32_pf<0>,
-        w6 ? (const void *) k_madj_f32_pf<6> : (const void *) k_madj_f32_pf<0>};
+        PF_KERNEL(k_fwd_f32_pf),
+        PF_KERNEL(k_adj_f32_pf),
+        PF_KERNEL(k_fwd_f64_pf),
+        PF_KERNEL(k_adj_f64_pf),
+        PF_KERNEL(k_fwd_madj_f32_pf),
+        PF_KERNEL(k_gadj_f32_pf),
+        PF_KERNEL(k_madj_f32_pf)};
+#undef PF_KERNEL
     static_assert(sizeof(pfKern) / sizeof(pfKern[0]) == PF_COUNT, "one kernel per PfKernel");
     static_assert(PF_COUNT <= (int) (sizeof(m->prefetchWave) / sizeof(m->prefetchWave[0])), "room for every wave");
     // block sizes: 64 threads (TileBlock) for the forward kernels and the
     // FP32 adjoint, 256 (one tile) for the FP64 adjoint and the adjoint parts
     const int pfBlock[PF_COUNT] = {CUPCFD_FWD_BLOCK,      CUPCFD_FWD_BLOCK, CUPCFD_FWD_BLOCK, TILE_CELLS,
-                                   CUPCFD_FWD_MADJ_BLOCK, TILE_CELLS,       TILE_CELLS};
+                                   CUPCFD_FWD_MADJ_BLOCK, CUPCFD_GADJ_BLOCK, TILE_CELLS};
     // prefetch distance in waves, in quarters, measured at 256^3 (same box):
     // 1.25 waves for the forward+mass adjoint (0.538 ms against 0.546 at 1
     // wave, 0.541 at 1.5, 0.581 at 0.75), the separate FP32 forward and
@@ -195,8 +209,10 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
 
 PrefetchArgs prefetch_args(const cupcfd_gpu_mesh *m, int kernel = -1) {
     PrefetchArgs p;
-    p.desc = (const TileDesc *) m->tileDesc;
-    p.inc = m->sell.inc;
+    const bool runs = list_form(m) == -6;
+    p.desc = (const TileDesc *) (runs ? m->tileDescRuns : m->tileDesc);
+    p.inc = runs ? (const int2 *) m->sell.runs : m->sell.inc;
+    p.runHead = runs ? m->sell.runHead : nullptr;
     p.nC = m->nC;
     p.nF = m->nF;
     p.nTiles = m->nTiles;
@@ -588,7 +604,7 @@ extern "C" int cupcfd_gpu_dev_forward_adjoint(cupcfd_gpu_mesh *m, int32_t precis
         CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[1], m->outStream));
         {
             KTIMER("k_gadj_f32_pf", st);
-            CG_LAUNCH_PF(m, k_gadj_f32_pf, grid, st, m->nC, sell(m), m->fg32, (const float *) grad, 2.f,
+            CG_LAUNCH_PF_BLOCK(m, k_gadj_f32_pf, grid * (TILE_CELLS / CUPCFD_GADJ_BLOCK), CUPCFD_GADJ_BLOCK, st, m->nC, sell(m), m->fg32, (const float *) grad, 2.f,
                          (float *) phiBar, (float *) phiBBar, m->nC, pfg);
             CG_LAUNCHED();
         }
@@ -944,7 +960,7 @@ int launch_adj_part(const cupcfd_gpu_mesh *m, bool f64, const void *g, double hs
         (gradPart ? hscale == 2.0 && aligned16(g) : hscale == 0.0 && !g && aligned16(state) && aligned16(gface))) {
         kt.set_name(gradPart ? "k_gadj_f32_pf" : "k_madj_f32_pf");
         if (gradPart)
-            CG_LAUNCH_PF(m, k_gadj_f32_pf, grid, st, m->nC, sell(m), m->fg32, (const float *) g, 2.f,
+            CG_LAUNCH_PF_BLOCK(m, k_gadj_f32_pf, grid * (TILE_CELLS / CUPCFD_GADJ_BLOCK), CUPCFD_GADJ_BLOCK, st, m->nC, sell(m), m->fg32, (const float *) g, 2.f,
                          (float *) phiBar, (float *) phiBBar, m->nC, prefetch_args(m, PF_GADJ));
         else
             CG_LAUNCH_PF(m, k_madj_f32_pf, grid, st, m->nC, sell(m), m->fg32, (const float4 *) state,

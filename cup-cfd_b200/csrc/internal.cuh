@@ -61,6 +61,17 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// One slice's entry into the run form (below).
+struct __align__(16) RunHead {
+    unsigned starts;  // bit l: lane l starts a run
+    int first;        // index of the slice's first run
+    int alternating;  // 2: every face of the slice's cells is interior, and each cell is the second cell of its
+                      // first face, the first cell of its second, and so on (a row inside a generated grid: low
+                      // and high x, y, z faces in turn); 1: the same but for boundary faces among the first two
+                      // (the ends of such a row); else 0
+    int pad;
+};
+
 // Cell-incidence lists in SELL-32 layout: the cells of slice s (internal ids
 // 32s .. 32s+31) own entries [slicePtr[s], slicePtr[s+1]); entry k of lane l
 // sits at slicePtr[s] + 32k + l, so entry k of a warp's 32 cells is one
@@ -77,6 +88,17 @@ struct Sell {
     int2 *inc = nullptr;
     int64_t nEntries = 0;
     int width = 0;  // the common width when every slice has it (then slice s starts at 32 * width * s), else 0
+    // Run form of lists six entries wide without padding (all hexahedral
+    // meshes), built where it is much shorter than inc. Along a row of cells
+    // numbered one after the other, each of the six faces, and the cell or
+    // boundary behind it, also advances by one: lane l's entries are lane l-1's
+    // with every face and other cell (boundary id) one higher. A run is a
+    // longest such stretch of a slice's lanes, stored as its first lane's six
+    // entries (48 bytes). A row inside the mesh takes two runs per slice (its
+    // first lane's low-x face belongs to the slice before).
+    RunHead *runHead = nullptr;
+    int4 *runs = nullptr;  // three per run
+    int nRuns = 0;
 };
 
 }  // namespace cupcfd_gpu
@@ -144,6 +166,7 @@ struct cupcfd_gpu_mesh {
     // L2-prefetch face loops: per-tile ranges (TileDesc[nTiles], 256-cell
     // tiles); tiles false when the faces are not numbered by owner tile
     void *tileDesc = nullptr;
+    void *tileDescRuns = nullptr;  // the same with the run form's ranges as the entry ranges
     int nTiles = 0;
     bool tiles = false;
     int prefetchDist = 0;         // tiles ahead for the L2 prefetch
@@ -183,6 +206,8 @@ struct Source {
     double *cc, *vol;                   // [3*nC], [nC]
 };
 int build_mesh_from_source(cupcfd_gpu_mesh *m, const Source &src, const cupcfd_mesh_options *opt);
+// run form of the incidence lists where it pays (mesh.cu)
+int build_runs(cupcfd_gpu_mesh *m, cudaStream_t st);
 // bandwidth of the numbering and the fused pipeline's device state (api.cu)
 int mesh_post_build(cupcfd_gpu_mesh *m, cudaStream_t st);
 int make_device_current(int device);

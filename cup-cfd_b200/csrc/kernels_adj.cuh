@@ -37,15 +37,14 @@ __device__ __forceinline__ double fwd_cell_f64(int c, const SellView &sv, const 
                                                const double *__restrict__ vol, const double *__restrict__ st,
                                                const double *__restrict__ gface, double *__restrict__ g,
                                                double *__restrict__ mflux, int64_t ldc) {
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
-    if (WF) w = WF;  // every cell has exactly WF entries (a full, uniform slice width)
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
     double phic = phi[c];
     double r0 = st[c], u0 = st[ldc + c], v0 = st[2 * ldc + c], w0 = st[3 * ldc + c];
     double ax = 0.0, ay = 0.0, az = 0.0, lsum = 0.0;
     for (int k0 = 0; k0 < w; k0 += CH) {
         int2 en[CH];
-        load_entries(e, k0, w, en);
+        e.load(k0, en);
         double4 G[CH];
         double pv[CH], so[CH][4], gf[CH];
 #pragma unroll
@@ -100,9 +99,8 @@ __device__ __forceinline__ double fwd_cell_f32(int c, const SellView &sv, const 
                                                const double *__restrict__ vol, const float4 *__restrict__ st,
                                                const float *__restrict__ gface, float *__restrict__ g,
                                                float *__restrict__ mflux, int64_t ldc) {
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
-    if (WF) w = WF;  // every cell has exactly WF entries (a full, uniform slice width)
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
     float phic = phi[c];
     float4 sc = st[c];
     Acc2x2 axy;  // (gx, gy) packed, gz alone
@@ -110,7 +108,7 @@ __device__ __forceinline__ double fwd_cell_f32(int c, const SellView &sv, const 
     double lsum = 0.0;
     for (int k0 = 0; k0 < w; k0 += CH) {
         int2 en[CH];
-        load_entries(e, k0, w, en);
+        e.load(k0, en);
         float4 G[CH], so[CH];
         float pv[CH], gf[CH];
 #pragma unroll
@@ -156,6 +154,57 @@ __device__ __forceinline__ double fwd_cell_f32(int c, const SellView &sv, const 
                     lsum);
 }
 
+// The seven compensated sums of fwd_madj_cell_f32, one face at a time.
+struct FwdMadjSums {
+    float phic;
+    float4 sc;
+    // in packed pairs: (gx, gy), (gz, rhobar), (ubar, vbar), wbar
+    Acc2x2 axy, azr, uvb;
+    Acc2 wb;
+    double lsum = 0.0;
+    __device__ __forceinline__ FwdMadjSums(float p, float4 s) : phic(p), sc(s) {}
+    __device__ __forceinline__ void boundary(const float4 &G, float pv) {
+        axy.add_prod(make_float2(pv, pv), make_float2(G.x, G.y));
+        azr.add_x(pv, G.z);
+    }
+    // ROLE: 0 / 1 this cell is the first / second cell of an interior face, -1 known from code and bnd only
+    template <int ROLE = -1>
+    __device__ __forceinline__ void add(int code, bool bnd, const float4 &G, float pv, const float4 &so, float gf,
+                                        float *__restrict__ mflux) {
+        if (ROLE < 0 && bnd) {
+            boundary(G, pv);
+            return;
+        }
+        const bool isN = ROLE < 0 ? code & 1 : ROLE;
+        const FaceW fw = face_weights(G.w, isN);
+        const float phif = interp(fw, phic, pv);
+        // rho_f and u_f . S_f from this cell's side: the owner's mass flux
+        // and this cell's mass-adjoint terms (adj_cell_f32)
+        const float4 sf = interp4(fw, sc, so);
+        const float q = udots(sf, G);
+        if (!isN) {
+            const float m = sf.x * q;
+            mflux[code >> 1] = m;
+            lsum = __fma_rn((double) gf, (double) m, lsum);
+        }
+        const float a = fw.wc * gf;
+        const float b = a * sf.x;
+        axy.add_prod(make_float2(phif, phif), make_float2(G.x, G.y));
+        azr.add_prod(make_float2(phif, a), make_float2(G.z, q));
+        uvb.add_prod(make_float2(b, b), make_float2(G.x, G.y));
+        wb.add_prod(b, G.z);
+    }
+    __device__ __forceinline__ double store(int c, double V, float *__restrict__ g, float4 *__restrict__ stbar,
+                                            int64_t ldc) const {
+        double fact = 1.0 / V;
+        float rx = (float) (axy.x() * fact), ry = (float) (axy.y() * fact), rz = (float) (azr.x() * fact);
+        g[c] = rx; g[ldc + c] = ry; g[2 * ldc + c] = rz;
+        stbar[c] = make_float4(azr.yf(), uvb.xf(), uvb.yf(), wb.value_f());
+        return __fma_rn(V, __fma_rn((double) rx, (double) rx, __fma_rn((double) ry, (double) ry, __dmul_rn((double) rz, (double) rz))),
+                        lsum);
+    }
+};
+
 // Per-cell body of the FP32 forward that also runs the mass-flux part of
 // the adjoint (which needs only inputs: state, gface and geometry): the
 // forward of fwd_cell_f32 plus, over every interior face, the rhobar / ubar
@@ -168,17 +217,11 @@ __device__ __forceinline__ double fwd_madj_cell_f32(int c, const SellView &sv, c
                                                     const float *__restrict__ gface, float *__restrict__ g,
                                                     float *__restrict__ mflux, float4 *__restrict__ stbar,
                                                     int64_t ldc) {
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
-    if (WF) w = WF;  // every cell has exactly WF entries (a full, uniform slice width)
-    float phic = phi[c];
-    float4 sc = st[c];
-    // seven compensated sums in packed pairs: (gx, gy), (gz, rhobar), (ubar, vbar), wbar
-    Acc2x2 axy, azr, uvb;
-    Acc2 wb;
-    double lsum = 0.0;
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
+    FwdMadjSums a(phi[c], st[c]);
     int2 en[CH];
-    load_entries(e, 0, w, en);
+    e.load(0, en);
     for (int k0 = 0; k0 < w; k0 += CH) {
         float4 G[CH], so[CH];
         float pv[CH], gf[CH];
@@ -195,47 +238,84 @@ __device__ __forceinline__ double fwd_madj_cell_f32(int c, const SellView &sv, c
             }
         }
         int2 nx[CH];
-        if (PIPE) load_entries(e, k0 + CH, w, nx);
+        if (PIPE) e.load(k0 + CH, nx);
 #pragma unroll
         for (int j = 0; j < CH; j++) {
             int code = en[j].x;
             if (!WF && code < 0) continue;
-            bool isN = code & 1;
-            int o = en[j].y;
-            float phif;
-            if (o < 0) {
-                phif = pv[j];
-                axy.add_prod(make_float2(phif, phif), make_float2(G[j].x, G[j].y));
-                azr.add_x(phif, G[j].z);
-            } else {
-                const FaceW fw = face_weights(G[j].w, isN);
-                phif = interp(fw, phic, pv[j]);
-                // rho_f and u_f . S_f from this cell's side: the owner's mass
-                // flux and this cell's mass-adjoint terms (adj_cell_f32)
-                const float4 sf = interp4(fw, sc, so[j]);
-                const float q = udots(sf, G[j]);
-                if (!isN) {
-                    const float m = sf.x * q;
-                    mflux[code >> 1] = m;
-                    lsum = __fma_rn((double) gf[j], (double) m, lsum);
-                }
-                const float a = fw.wc * gf[j];
-                const float b = a * sf.x;
-                axy.add_prod(make_float2(phif, phif), make_float2(G[j].x, G[j].y));
-                azr.add_prod(make_float2(phif, a), make_float2(G[j].z, q));
-                uvb.add_prod(make_float2(b, b), make_float2(G[j].x, G[j].y));
-                wb.add_prod(b, G[j].z);
-            }
+            a.add(code, en[j].y < 0, G[j], pv[j], so[j], gf[j], mflux);
         }
-        next_entries<PIPE>(e, k0 + CH, w, en, nx);
+        next_entries<PIPE>(e, k0 + CH, en, nx);
     }
-    double V = vol[c];
-    double fact = 1.0 / V;
-    float rx = (float) (axy.x() * fact), ry = (float) (axy.y() * fact), rz = (float) (azr.x() * fact);
-    g[c] = rx; g[ldc + c] = ry; g[2 * ldc + c] = rz;
-    stbar[c] = make_float4(azr.yf(), uvb.xf(), uvb.yf(), wb.value_f());
-    return __fma_rn(V, __fma_rn((double) rx, (double) rx, __fma_rn((double) ry, (double) ry, __dmul_rn((double) rz, (double) rz))),
-                    lsum);
+    return a.store(c, vol[c], g, stbar, ldc);
+}
+
+// The same for lists in run form, with the faces past the first
+// CUPCFD_STAGE_FROM gathered into shared memory by cp.async before the first
+// ones' arithmetic. ALT: the slice's RunHead::alternating (with 2 no face is a
+// boundary's and every role is known, with 1 past the first two).
+template <int BLOCK>
+struct FwdMadjStage {
+    static constexpr int N = 6 - CUPCFD_STAGE_FROM;
+    float4 G[N][BLOCK], so[N][BLOCK];
+    float pv[N][BLOCK], gf[N][BLOCK];
+};
+template <int ALT, int BLOCK>
+__device__ __forceinline__ double fwd_madj_cell_staged(int c, const CellList<-6> &e, FwdMadjStage<BLOCK> &sh,
+                                                       const float4 *__restrict__ fg, const float *__restrict__ phi,
+                                                       const float *__restrict__ phiB, const double *__restrict__ vol,
+                                                       const float4 *__restrict__ st, const float *__restrict__ gface,
+                                                       float *__restrict__ g, float *__restrict__ mflux,
+                                                       float4 *__restrict__ stbar, int64_t ldc) {
+    constexpr int N = 6, D = CUPCFD_STAGE_FROM;
+    const int t = threadIdx.x;
+    int code[N], other[N];  // ALT: the face itself in place of the code
+    if (ALT) {
+        e.template load_alternating<ALT>(code, other);
+    } else {
+        int2 en[N];
+        e.load(0, en);
+#pragma unroll
+        for (int j = 0; j < N; j++) { code[j] = en[j].x; other[j] = en[j].y; }
+    }
+#pragma unroll
+    for (int j = D; j < N; j++) {
+        const int f = ALT ? code[j] : code[j] >> 1, o = other[j];
+        stage16(&sh.G[j - D][t], fg + f);
+        stage4(&sh.pv[j - D][t], ALT > (j < 2 ? 1 : 0) || o >= 0 ? phi + o : phiB + (-1 - o));
+        if (ALT > (j < 2 ? 1 : 0) || o >= 0) {
+            stage16(&sh.so[j - D][t], st + o);
+            stage4(&sh.gf[j - D][t], gface + f);
+        }
+        if ((j - D) % 2 == 1) stage_commit();
+    }
+    FwdMadjSums a(phi[c], st[c]);
+    float4 G[D + 1], so[D + 1];
+    float pv[D + 1], gf[D + 1];
+#pragma unroll
+    for (int j = 0; j < D; j++) {
+        const int f = ALT ? code[j] : code[j] >> 1, o = other[j];
+        G[j] = __ldg(fg + f);
+        pv[j] = ALT > (j < 2 ? 1 : 0) || o >= 0 ? __ldg(phi + o) : __ldg(phiB + (-1 - o));
+        if (ALT > (j < 2 ? 1 : 0) || o >= 0) {
+            so[j] = __ldg(st + o);
+            gf[j] = __ldg(gface + f);
+        }
+    }
+    auto add = [&](int j, const float4 &G, float pv, const float4 &so, float gf) {
+        if (!ALT) a.add(code[j], other[j] < 0, G, pv, so, gf, mflux);
+        else if (ALT == 1 && j < 2 && other[j] < 0) a.boundary(G, pv);
+        else if (j % 2) a.template add<0>(2 * code[j], false, G, pv, so, gf, mflux);
+        else a.template add<1>(0, false, G, pv, so, gf, mflux);
+    };
+#pragma unroll
+    for (int j = 0; j < D; j++) add(j, G[j], pv[j], so[j], gf[j]);
+#pragma unroll
+    for (int j = D; j < N; j++) {
+        if ((j - D) % 2 == 0) stage_wait((N - j) / 2 - 1);
+        add(j, sh.G[j - D][t], sh.pv[j - D][t], sh.so[j - D][t], sh.gf[j - D][t]);
+    }
+    return a.store(c, vol[c], g, stbar, ldc);
 }
 
 // ---------------------------------------------------------------------------
@@ -382,9 +462,8 @@ __device__ __forceinline__ void adj_cell_f64(int c, const SellView &sv, const do
                                              const double *g, double hscale, const double *__restrict__ st,
                                              const double *__restrict__ gface, double *__restrict__ phibar,
                                              double *__restrict__ phibBar, double *__restrict__ stbar, int64_t ldc) {
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
-    if (WF) w = WF;  // every cell has exactly WF entries (a full, uniform slice width)
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
     bool doG = hscale != 0.0, doM = gface != nullptr;
     double hx = 0, hy = 0, hz = 0;
     if (doG) { hx = hscale * ldg_g<LDCG>(g + c); hy = hscale * ldg_g<LDCG>(g + ldc + c); hz = hscale * ldg_g<LDCG>(g + 2 * ldc + c); }
@@ -393,7 +472,7 @@ __device__ __forceinline__ void adj_cell_f64(int c, const SellView &sv, const do
     double pb = 0.0, rb = 0.0, ub = 0.0, vb = 0.0, wb = 0.0;
     for (int k0 = 0; k0 < w; k0 += CH) {
         int2 en[CH];
-        load_entries(e, k0, w, en);
+        e.load(k0, en);
         double4 G[CH];
         double go[CH][3], so[CH][4], gf[CH];
 #pragma unroll
@@ -448,9 +527,8 @@ __device__ __forceinline__ void adj_cell_f32(int c, const SellView &sv, const fl
                                              float hscale, const float4 *__restrict__ st,
                                              const float *__restrict__ gface, float *__restrict__ phibar,
                                              float *__restrict__ phibBar, float4 *__restrict__ stbar, int64_t ldc) {
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
-    if (WF) w = WF;  // every cell has exactly WF entries (a full, uniform slice width)
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
     bool doG = hscale != 0.f, doM = gface != nullptr;
     float hx = 0, hy = 0, hz = 0;
     if (doG) { hx = hscale * ldg_g<LDCG>(g + c); hy = hscale * ldg_g<LDCG>(g + ldc + c); hz = hscale * ldg_g<LDCG>(g + 2 * ldc + c); }
@@ -459,7 +537,7 @@ __device__ __forceinline__ void adj_cell_f32(int c, const SellView &sv, const fl
     Acc2 pb, rb, wb;
     Acc2x2 uvb;  // (ubar, vbar) packed
     int2 en[CH];
-    load_entries(e, 0, w, en);
+    e.load(0, en);
     for (int k0 = 0; k0 < w; k0 += CH) {
         float4 G[CH], so[CH];
         float go[CH][3], gf[CH];
@@ -474,7 +552,7 @@ __device__ __forceinline__ void adj_cell_f32(int c, const SellView &sv, const fl
             if (doM) { so[j] = __ldg(st + o); gf[j] = __ldg(gface + f); }
         }
         int2 nx[CH];
-        if (PIPE) load_entries(e, k0 + CH, w, nx);
+        if (PIPE) e.load(k0 + CH, nx);
 #pragma unroll
         for (int j = 0; j < CH; j++) {
             int code = en[j].x;
@@ -498,10 +576,79 @@ __device__ __forceinline__ void adj_cell_f32(int c, const SellView &sv, const fl
                 wb.add_prod(b, G[j].z);
             }
         }
-        next_entries<PIPE>(e, k0 + CH, w, en, nx);
+        next_entries<PIPE>(e, k0 + CH, en, nx);
     }
     if (doG) phibar[c] = pb.value_f();
     if (doM) stbar[c] = make_float4(rb.value_f(), uvb.xf(), uvb.yf(), wb.value_f());
+}
+
+// The gradient part of adj_cell_f32 for six-entry lists, with the faces past
+// the first CUPCFD_GADJ_STAGE_FROM gathered into shared memory (cp.async)
+// before the first ones' arithmetic; the same sums in the same order.
+#ifndef CUPCFD_GADJ_STAGE_FROM
+#define CUPCFD_GADJ_STAGE_FROM 2
+#endif
+template <int BLOCK>
+struct GadjStage {
+    static constexpr int N = 6 - CUPCFD_GADJ_STAGE_FROM;
+    float4 G[N][BLOCK];
+    float g[N][3][BLOCK];
+};
+template <int ALT, int BLOCK>
+__device__ __forceinline__ void gadj_cell_staged(int c, const CellList<-6> &e, GadjStage<BLOCK> &sh,
+                                                 const float4 *__restrict__ fg, const float *__restrict__ g, float hscale,
+                                                 float *__restrict__ phibar, float *__restrict__ phibBar, int64_t ldc) {
+    constexpr int N = 6, D = CUPCFD_GADJ_STAGE_FROM;
+    const int t = threadIdx.x;
+    int code[N], other[N];  // ALT: the face itself in place of the code
+    if (ALT) {
+        e.template load_alternating<ALT>(code, other);
+    } else {
+        int2 en[N];
+        e.load(0, en);
+#pragma unroll
+        for (int j = 0; j < N; j++) { code[j] = en[j].x; other[j] = en[j].y; }
+    }
+#pragma unroll
+    for (int j = D; j < N; j++) {
+        const int o = other[j];
+        stage16(&sh.G[j - D][t], fg + (ALT ? code[j] : code[j] >> 1));
+        if (ALT > (j < 2 ? 1 : 0) || o >= 0) {
+            stage4(&sh.g[j - D][0][t], g + o);
+            stage4(&sh.g[j - D][1][t], g + ldc + o);
+            stage4(&sh.g[j - D][2][t], g + 2 * ldc + o);
+        }
+        if ((j - D) % 2 == 1) stage_commit();
+    }
+    const float hx = hscale * __ldg(g + c), hy = hscale * __ldg(g + ldc + c), hz = hscale * __ldg(g + 2 * ldc + c);
+    float4 G[D + 1];
+    float go[D + 1][3];
+#pragma unroll
+    for (int j = 0; j < D; j++) {
+        const int o = other[j];
+        G[j] = __ldg(fg + (ALT ? code[j] : code[j] >> 1));
+        if (ALT > (j < 2 ? 1 : 0) || o >= 0) {
+            go[j][0] = __ldg(g + o); go[j][1] = __ldg(g + ldc + o); go[j][2] = __ldg(g + 2 * ldc + o);
+        }
+    }
+    Acc2 pb;
+    auto add = [&](int j, const float4 &G, float g0, float g1, float g2) {
+        if (ALT < (j < 2 ? 2 : 1) && other[j] < 0) {
+            phibBar[-1 - other[j]] = fmaf(hx, G.x, fmaf(hy, G.y, hz * G.z));
+            return;
+        }
+        const FaceW fw = face_weights(G.w, ALT ? j % 2 == 0 : code[j] & 1);
+        const float sx = fmaf(hscale, g0, hx), sy = fmaf(hscale, g1, hy), sz = fmaf(hscale, g2, hz);
+        pb.add_prod(fw.wc, fmaf(sx, G.x, fmaf(sy, G.y, sz * G.z)));
+    };
+#pragma unroll
+    for (int j = 0; j < D; j++) add(j, G[j], go[j][0], go[j][1], go[j][2]);
+#pragma unroll
+    for (int j = D; j < N; j++) {
+        if ((j - D) % 2 == 0) stage_wait((N - j) / 2 - 1);
+        add(j, sh.G[j - D][t], sh.g[j - D][0][t], sh.g[j - D][1][t], sh.g[j - D][2][t]);
+    }
+    phibar[c] = pb.value_f();
 }
 
 __global__ void __launch_bounds__(256, CUPCFD_MINB_ADJ_F64) k_adj_f64(int nC, SellView sv, const double4 *__restrict__ fg,

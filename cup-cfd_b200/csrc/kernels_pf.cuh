@@ -20,7 +20,7 @@ namespace cupcfd_gpu {
 // ahead (cp.async.bulk.prefetch.L2). Shared memory and L1 are untouched;
 // the streamed loads of later blocks become L2 hits.
 //
-// WF: 0 for any mesh; 6 when every cell has exactly six incidences (all
+// WF: 0 for any mesh; -6 lists in run form (CellList in sell.cuh); 6 when every cell has exactly six incidences (all
 // hexahedral meshes: every slice six entries wide, no padding). The cell
 // loop then has a compile-time trip count: no padding checks, the chunks
 // unrolled and their loads scheduled across chunks (same arithmetic in the
@@ -123,6 +123,15 @@ __global__ void __launch_bounds__(TILE_CELLS, CUPCFD_MINB_ADJ_F64)
 // warp k of tile t at lossPart[k nTiles + t]; k_reduce_partials<8> sums each
 // tile's eight in order, which gives the per-tile value of
 // block_sum_store<256> bit for bit.
+//
+// On lists in run form (WF -6) the faces past the first two are gathered into
+// shared memory (fwd_madj_cell_staged; 10 KB a block, 160 KB an SM) at the same
+// 64 registers and 32 warps per SM. At 256^3, 50-step runs on one box:
+// 0.480-0.485 ms against 0.540 with the lists and gathers of two faces at a
+// time; the run form alone 0.555, and roles known at compile time cut its
+// instructions from 752 to about 620 a warp (0.83 against 0.86 ms for the
+// step under the power limit). Five tiles a SM (48 registers) 0.567, three
+// (24 warps) 0.54. It moves 2.07 GB, at 4.3 TB/s; issue slots are 60-70% busy.
 #ifndef CUPCFD_FWD_MADJ_CHUNK
 #define CUPCFD_FWD_MADJ_CHUNK 2
 #endif
@@ -146,7 +155,16 @@ __global__ void __launch_bounds__(CUPCFD_FWD_MADJ_BLOCK, CUPCFD_MINB_FWD_MADJ *T
     const int cellBytes[3] = {T * 4, T * 16, T * 8};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     double l = 0.0;
-    if (c < nC) l = fwd_madj_cell_f32<CUPCFD_FWD_MADJ_CHUNK, 0, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc);
+    if (c < nC) {
+        if constexpr (WF == -6) {
+            __shared__ FwdMadjStage<CUPCFD_FWD_MADJ_BLOCK> stage;
+            const CellList<WF> e(sv, c);
+            l = e.alternating == 2   ? fwd_madj_cell_staged<2>(c, e, stage, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc)
+                : e.alternating == 1 ? fwd_madj_cell_staged<1>(c, e, stage, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc)
+                                     : fwd_madj_cell_staged<0>(c, e, stage, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc);
+        } else
+            l = fwd_madj_cell_f32<CUPCFD_FWD_MADJ_CHUNK, 0, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc);
+    }
     if (tb.lead) prefetch_tile<3>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
     if (lossPart) warp_partial_store<CUPCFD_FWD_MADJ_BLOCK>(l, c, lossPart);
 }
@@ -155,28 +173,42 @@ __global__ void __launch_bounds__(CUPCFD_FWD_MADJ_BLOCK, CUPCFD_MINB_FWD_MADJ *T
 // phibar and phibBar. The next chunk's entries load during the current
 // chunk's arithmetic (CUPCFD_GADJ_PIPE) within the 40 registers that six
 // resident blocks per SM leave (CUPCFD_MINB_GADJ): chosen by measurement.
+// On lists in run form it stages the gradients and face records of four faces
+// (gadj_cell_staged, 7 KB a block) in 64-thread blocks: 0.237-0.249 ms against
+// 0.278 at 256^3 (256-thread blocks 0.250, five tiles an SM 0.255-0.269, eight
+// 0.314), 1.14 GB of DRAM traffic against 1.86.
 #ifndef CUPCFD_GADJ_PIPE
 #define CUPCFD_GADJ_PIPE 1
 #endif
 #ifndef CUPCFD_MINB_GADJ
 #define CUPCFD_MINB_GADJ 6
 #endif
+#ifndef CUPCFD_GADJ_BLOCK
+#define CUPCFD_GADJ_BLOCK 64
+#endif
 template <int WF>
-__global__ void __launch_bounds__(TILE_CELLS, CUPCFD_MINB_GADJ)
+__global__ void __launch_bounds__(CUPCFD_GADJ_BLOCK, CUPCFD_MINB_GADJ *TILE_CELLS / CUPCFD_GADJ_BLOCK)
     k_gadj_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ g, float hscale,
                   float *__restrict__ phibar, float *__restrict__ phibBar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    int c = blockIdx.x * T + threadIdx.x;
-    const int tp = blockIdx.x + pf.dist;
-    const bool lead = threadIdx.x == T - 32 && tp < pf.nTiles;
+    const TileBlock<CUPCFD_GADJ_BLOCK> tb(pf);
+    const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[3] = {g, g + ldc, g + 2 * ldc};
     const int cellBytes[3] = {T * 4, T * 4, T * 4};
-    if (lead) fetch_ranges_async(&s_rng, pf.desc + tp);
-    if (c < nC)
-        adj_cell_f32<false, CUPCFD_ADJ_CHUNK, CUPCFD_GADJ_PIPE, WF>(c, sv, fg, g, hscale, nullptr, nullptr, phibar,
-                                                                phibBar, nullptr, ldc);
-    if (lead) prefetch_tile<3>(pf, tp, ranges_ready(&s_rng), fg, 16, (const float *) nullptr, cellSrc, cellBytes);
+    if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
+    if (c < nC) {
+        if constexpr (WF == -6) {
+            __shared__ GadjStage<CUPCFD_GADJ_BLOCK> stage;
+            const CellList<WF> e(sv, c);
+            if (e.alternating == 2) gadj_cell_staged<2>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
+            else if (e.alternating == 1) gadj_cell_staged<1>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
+            else gadj_cell_staged<0>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
+        } else
+            adj_cell_f32<false, CUPCFD_ADJ_CHUNK, CUPCFD_GADJ_PIPE, WF>(c, sv, fg, g, hscale, nullptr, nullptr, phibar,
+                                                                    phibBar, nullptr, ldc);
+    }
+    if (tb.lead) prefetch_tile<3>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, (const float *) nullptr, cellSrc, cellBytes);
 }
 
 // Mass-flux part of the adjoint only (adj_cell_f32 with hscale 0): stbar
@@ -259,6 +291,19 @@ __global__ void k_tile_desc(int nTiles, int nSlices, const int *__restrict__ sli
     atomicMax(maxima + 0, d.entEnd - d.entStart);
     atomicMax(maxima + 1, d.fe - d.fs);
     atomicMax(maxima + 2, wmax);
+}
+
+// The descriptors of the run form: the same tiles, with the range of the
+// tile's runs (six int2 each) in place of its SELL entries.
+__global__ void k_tile_desc_runs(int nTiles, int nSlices, int nRuns, const RunHead *__restrict__ runHead,
+                                 const TileDesc *__restrict__ desc, TileDesc *__restrict__ out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nTiles) return;
+    const int s0 = t * (TILE_CELLS / 32), s1 = s0 + TILE_CELLS / 32;
+    TileDesc d = desc[t];
+    d.entStart = 6 * runHead[s0].first;
+    d.entEnd = 6 * (s1 < nSlices ? runHead[s1].first : nRuns);
+    out[t] = d;
 }
 
 }  // namespace cupcfd_gpu

@@ -30,7 +30,8 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned) 
 
 struct PrefetchArgs {
     const TileDesc *desc;
-    const int2 *inc;
+    const int2 *inc;      // what desc's entry ranges index: the SELL entries, or the runs' (struct Sell)
+    const RunHead *runHead;  // run form: the slices' heads, else null
     int nC, nF, nTiles, dist;
 };
 
@@ -90,6 +91,7 @@ __device__ __forceinline__ void prefetch_tile(const PrefetchArgs &p, int t, cons
                                               const int (&cellBytes)[NCELL]) {
     constexpr int PER16 = 16 / (int) sizeof(TG);
     const int entStart = d.x, entEnd = d.y, fs = d.z, fe = d.w;
+    if (p.runHead) bulk_prefetch_l2(p.runHead + (size_t) t * (TILE_CELLS / 32), TILE_CELLS / 32 * (unsigned) sizeof(RunHead));
     if (entEnd > entStart) bulk_prefetch_l2(p.inc + entStart, (unsigned) (entEnd - entStart) * 8u);
     if (fe > fs)
         bulk_prefetch_l2(static_cast<const unsigned char *>(fg) + (size_t) fs * fgSize, (unsigned) (fe - fs) * (unsigned) fgSize);

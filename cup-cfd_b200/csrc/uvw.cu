@@ -112,7 +112,7 @@ int run_face_loop(cupcfd_gpu_mesh *m, T gammaBlend, T small, const T *u, const T
     CG_TRY(ensure_state(m, st));
     UvwArgs<T> a;
     a.nC = m->nC;
-    a.sv = SellView{m->sell.slicePtr, m->sell.inc, m->sell.width};
+    a.sv = SellView{m->sell.slicePtr, m->sell.inc, m->sell.width, m->sell.runHead, m->sell.runs};
     a.fcells = m->faceCells;
     if constexpr (F64) {
         a.fg = m->fg64; a.fc = m->fc64; a.cc = m->cc64;
@@ -142,6 +142,7 @@ int run_face_loop(cupcfd_gpu_mesh *m, T gammaBlend, T small, const T *u, const T
         PrefetchArgs pf;
         pf.desc = (const TileDesc *) m->tileDesc;
         pf.inc = m->sell.inc;
+        pf.runHead = nullptr;
         pf.nC = m->nC;
         pf.nF = m->nF;
         pf.nTiles = m->nTiles;

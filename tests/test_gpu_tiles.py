@@ -289,3 +289,47 @@ def test_fp64_forward_prefetch_equals_plain(cg, gpu):
     assert {"k_fwd_f64_pf", "k_adj_f64_pf"} <= out[0][-1] and {"k_fwd_f64", "k_adj_f64"} <= out[1][-1]
     for a, b in zip(out[0][:-1], out[1][:-1]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dims", [(32, 6, 5),     # one slice per row: low and high x boundary in every slice
+                                  (64, 8, 6),     # slices at one end of a row, interior rows
+                                  (33, 12, 7),    # rows break inside slices, odd cell count, ragged last slice
+                                  (100, 7, 8),    # several breaks per slice
+                                  (257, 3, 4)])   # one cell past a tile
+def test_run_form_equals_lists(cg, gpu, dims, monkeypatch):
+    """Rows of cells numbered one after the other store their incidence lists
+    in run form (one entry set per stretch of lanes); the kernels that read it
+    give the bits of those that read the full lists (CUPCFD_RUNS=0 at mesh
+    creation), FP32 and FP64."""
+    import torch
+    monkeypatch.setenv("CUPCFD_RUNS", "0")
+    lists = cg.Mesh.structgen(*dims, order=cg.ORDER_OWNER)
+    monkeypatch.delenv("CUPCFD_RUNS")
+    runs = cg.Mesh.structgen(*dims, order=cg.ORDER_OWNER)
+    assert lists.full_width == 6 and runs.full_width == 6
+    assert runs.deviceBytes > lists.deviceBytes, "the run form was not built"
+    fields = _fields(torch, runs, 17)
+    _assert_same(_run_pipeline(cg, torch, runs, *fields, offset=False),
+                 _run_pipeline(cg, torch, lists, *fields, offset=False))
+    _assert_same(_run(cg, torch, runs, *fields, offset=False), _run(cg, torch, lists, *fields, offset=False))
+    phi, phiB, st, gface = (t.double() for t in fields)
+    st = st.t().contiguous()
+    outs = []
+    for mesh in (runs, lists):
+        e = lambda *n: torch.full(n, float("nan"), dtype=torch.float64, device="cuda:0")
+        o = [e(3, mesh.nCells), torch.zeros_like(gface), e(1), e(mesh.nCells), e(mesh.nBoundaries), e(4, mesh.nCells)]
+        s = torch.cuda.current_stream()
+        cg.dev_forward(mesh, cg.PREC_F64, phi, phiB, st, o[0], o[1], gface=gface, loss=o[2], stream=s)
+        cg.dev_adjoint(mesh, cg.PREC_F64, o[0], st, gface, o[3], o[4], o[5], stream=s)
+        mesh.check_status()
+        torch.cuda.synchronize()
+        outs.append(o)
+    _assert_same(*outs)
+
+
+def test_irregular_numbering_has_no_run_form(cg, gpu, monkeypatch):
+    """A permuted mesh has no stretches worth storing and keeps the lists."""
+    monkeypatch.setenv("CUPCFD_RUNS", "0")
+    lists = cg.Mesh.jittered(20, 18, 16, order=cg.ORDER_OWNER)
+    monkeypatch.delenv("CUPCFD_RUNS")
+    assert cg.Mesh.jittered(20, 18, 16, order=cg.ORDER_OWNER).deviceBytes == lists.deviceBytes
