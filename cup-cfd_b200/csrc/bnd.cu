@@ -18,15 +18,20 @@ namespace {
 
 constexpr int BT = 256;
 // scratch slots of the host-buffer calls (kept across calls)
-enum BndSlot { B_MF = 40, B_SU, B_U, B_V, B_W, B_DEN, B_REG, B_REG2, B_SCAL, B_SELC, B_SELV, B_SELR, B_STAGE };
+enum BndSlot { B_MF = 40, B_SU, B_U, B_V, B_W, B_DEN, B_REG, B_REG2, B_SCAL, B_VALS, B_STAGE };
 
 // Boundary -> face and sorted-boundary -> cell maps for the caller's numbering.
+// list: the faces of the boundaries grouped by type (BndLists).
 struct Maps {
-    const int *face, *cell;
+    const int *face, *cell, *list;
 };
 inline Maps maps_for(const cupcfd_gpu_mesh *m, bool internal) {
-    return internal ? Maps{m->bndFaceInt, m->bndSortedCellInt} : Maps{m->bndFaceRef, m->bndSortedCellRef};
+    return internal ? Maps{m->bndFaceInt, m->bndSortedCellInt, m->bndLists.faceInt}
+                    : Maps{m->bndFaceRef, m->bndSortedCellRef, m->bndLists.faceRef};
 }
+
+// Scratch for the values of a type's boundaries.
+int values(cupcfd_gpu_mesh *m, double **vals);
 
 int check_mesh(const cupcfd_gpu_mesh *m, bool needGeometry) {
     CG_RETURN_IF(!m, CUPCFD_E_NULL_PTR, "boundary loop: null mesh");
@@ -54,6 +59,8 @@ int down(void *h, const void *d, size_t bytes, cudaStream_t st) {
     return CUPCFD_E_SUCCESS;
 }
 
+int values(cupcfd_gpu_mesh *m, double **vals) { return slot(m, B_VALS, m->nB, vals); }
+
 // Float host arrays go through one float staging buffer, sized once per call
 // for its longest array (the copies and conversions are stream-ordered, so
 // every array of a call can use it in turn).
@@ -80,38 +87,29 @@ int down_real(float *stage, H *h, const double *d, size_t n, cudaStream_t st) {
     return down(h, stage, sizeof(float) * n, st);
 }
 
-// The sum over the boundaries of region type `type`, in boundary order, of
-// base[map[ib] * stride + offset], from *init (or initValue) into *out, and
-// into regionAcc[region] (may be null) in the same order.
-template <bool F32>
-int ordered_sum(cupcfd_gpu_mesh *m, int type, const double *base, int stride, int offset, const int *map,
-                const double *init, double initValue, double *out, double *regionAcc, cudaStream_t st) {
-    int *cnt, *regs;
-    double *vals;
-    CG_TRY(slot(m, B_SELC, (size_t) m->nB / SEL_T + 2, &cnt));
-    CG_TRY(slot(m, B_SELV, (size_t) m->nB, &vals));
-    CG_TRY(slot(m, B_SELR, (size_t) m->nB, &regs));
-    return launch_ordered_sum<1, F32>(SelArgs{m->nB, m->bndRegion, m->regionType, type}, base, stride, offset, map, init,
-                                 initValue, out, regionAcc, m->nR, cnt, vals, regs, st);
-}
-
 // ---- the loops on device arrays (face arrays indexed through mp.face, cell
 // arrays through mp.cell); every scalar in device memory ----
 template <bool F32>
 int run_loop1(cupcfd_gpu_mesh *m, Maps mp, const double *mf, double *flowin, cudaStream_t st) {
-    return ordered_sum<F32>(m, CUPCFD_RTYPE_INLET, mf, 1, 0, mp.face, nullptr, 0.0, flowin, nullptr, st);
+    double *vals;
+    CG_TRY(values(m, &vals));
+    return launch_gathered_sum<F32>(m, CUPCFD_RTYPE_INLET, mp.list, mf, 1, 0, 1, vals, flowin, nullptr, st);
 }
 
 template <bool F32>
 int run_loop2(cupcfd_gpu_mesh *m, Maps mp, const double *mf, double *flowRegion, double *flowout, cudaStream_t st) {
-    return ordered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, mf, 1, 0, mp.face, nullptr, 0.0, flowout, flowRegion, st);
+    double *vals;
+    CG_TRY(values(m, &vals));
+    return launch_gathered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, mp.list, mf, 1, 0, 1, vals, flowout, flowRegion, st);
 }
 
 template <bool F32>
 int run_loop3(cupcfd_gpu_mesh *m, const double *flowin, double *ratearea, double *areaout, cudaStream_t st) {
     // face areas from the internal {xf, yf, zf, area} records
-    CG_TRY(ordered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, (const double *) m->fc64, 4, 3, m->bndFaceInt, nullptr, 0.0, areaout,
-                       nullptr, st));
+    double *vals;
+    CG_TRY(values(m, &vals));
+    CG_TRY(launch_gathered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, m->bndLists.faceInt, (const double *) m->fc64, 4, 3, 1, vals,
+                                    areaout, nullptr, st));
     k_bl_ratearea<F32><<<1, 1, 0, st>>>(flowin, areaout, ratearea);
     CG_LAUNCHED();
     return CUPCFD_E_SUCCESS;
@@ -120,27 +118,34 @@ int run_loop3(cupcfd_gpu_mesh *m, const double *flowin, double *ratearea, double
 template <bool F32>
 int run_loop4(cupcfd_gpu_mesh *m, Maps mp, double *mf, double *uB, double *vB, double *wB, const double *denB,
               const double *ratearea, double *flowout, cudaStream_t st) {
-    if (m->nB > 0) {
-        k_bl4_update<F32><<<grid_for(m->nB, BT), BT, 0, st>>>(m->nB, m->bndRegion, m->regionType, m->regionSplvl, mp.face,
-                                                         m->bndFaceInt, m->fg64, m->fc64, mf, uB, vB, wB, denB, ratearea);
+    const int n = m->bndLists.count(CUPCFD_RTYPE_OUTLET), s0 = m->bndLists.typeStart[CUPCFD_RTYPE_OUTLET];
+    double *vals;
+    CG_TRY(values(m, &vals));
+    if (n > 0) {
+        k_bl4_update<F32><<<grid_for(n, BT), BT, 0, st>>>(n, m->bndLists.id + s0, mp.list + s0, m->bndLists.faceInt + s0,
+                                                          m->bndRegion, m->regionSplvl, m->fg64, m->fc64, mf, uB, vB, wB,
+                                                          denB, ratearea, vals);
         CG_LAUNCHED();
     }
-    return ordered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, mf, 1, 0, mp.face, nullptr, 0.0, flowout, nullptr, st);
+    return launch_ordered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, vals, 1, nullptr, 0.0, flowout, nullptr, st);
 }
 
 template <bool F32>
 int run_loop5(cupcfd_gpu_mesh *m, Maps mp, double *mf, double *su, double *uB, double *vB, double *wB, double fact,
               int solveU, int solveV, int solveW, const double *flowFact, double *flowout2, cudaStream_t st) {
-    if (m->nB > 0) {
-        k_bl5_update<F32><<<grid_for(m->nB, BT), BT, 0, st>>>(m->nB, m->bndRegion, m->regionType, mp.face, mf, flowFact, uB,
-                                                         vB, wB, fact, solveU, solveV, solveW);
+    const int n = m->bndLists.count(CUPCFD_RTYPE_OUTLET), s0 = m->bndLists.typeStart[CUPCFD_RTYPE_OUTLET];
+    double *vals;
+    CG_TRY(values(m, &vals));
+    if (n > 0) {
+        k_bl5_update<F32><<<grid_for(n, BT), BT, 0, st>>>(n, m->bndLists.id + s0, mp.list + s0, m->bndRegion, mf, flowFact,
+                                                          uB, vB, wB, fact, solveU, solveV, solveW, vals);
         CG_LAUNCHED();
         k_bl5_su<F32><<<grid_for(m->nB, BT), BT, 0, st>>>(m->nB, m->bndSorted, mp.cell, m->bndRegion, m->regionType, mp.face,
                                                      mf, su);
         CG_LAUNCHED();
     }
     // *flowout2 is not reset (MassKernels.ipp:457-521): the sum starts from its value
-    return ordered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, mf, 1, 0, mp.face, flowout2, 0.0, flowout2, nullptr, st);
+    return launch_ordered_sum<F32>(m, CUPCFD_RTYPE_OUTLET, vals, 1, flowout2, 0.0, flowout2, nullptr, st);
 }
 
 template <bool F32>

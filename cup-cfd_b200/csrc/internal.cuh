@@ -101,6 +101,20 @@ struct Sell {
     int nRuns = 0;
 };
 
+// The boundaries in boundary order, grouped by region type (type t's from
+// typeStart[t]), as ids and as their faces in both numberings, and grouped by
+// region (region r's from regionStart[r]), as places in their type's list:
+// what the ordered sums walk. Built with the regions; the pointers are null
+// while every region is a default one.
+struct BndLists {
+    int *id = nullptr, *faceRef = nullptr, *faceInt = nullptr;
+    int *regionPlace = nullptr, *regionStart = nullptr;
+    int *storage = nullptr;  // [4 nB] behind the four lists
+    int regionCap = 0;       // regions regionStart has room for
+    int typeStart[6] = {};
+    int count(int type) const { return typeStart[type + 1] - typeStart[type]; }
+};
+
 }  // namespace cupcfd_gpu
 
 struct cupcfd_gpu_mesh {
@@ -151,6 +165,7 @@ struct cupcfd_gpu_mesh {
     int *bndFaceRef = nullptr, *bndFaceInt = nullptr;
     int *bndSorted = nullptr, *bndSortedCellInt = nullptr, *bndSortedCellRef = nullptr;
     bool bndMapsOk = false;
+    cupcfd_gpu::BndLists bndLists;
     std::vector<int> hRegionType;
     // momentum loops (FluxUVWDolfyn*): getFaceRLencos per internal face and
     // getBoundaryDistance per boundary (null = all zero until set), boundary

@@ -3,9 +3,9 @@
 //
 // The reference walks boundaries ib = 0 .. nB-1 and adds into scalars (and,
 // in loop 2, per-region sums) one boundary at a time; reproducing its
-// rounding means adding in that order (ordered_sum.cuh: the selected
-// boundaries gathered in parallel, then one chain of additions per sum). The per-boundary updates
-// (loops 4 and 5) are independent and run one thread per boundary. Loop 5's
+// rounding means the sums of additions in that order (ordered_sum.cuh). The
+// per-boundary updates (loops 4 and 5) are independent and run one thread per
+// outlet boundary. Loop 5's
 // su[cell1] -= massFlux applies, per cell, its outlet boundaries in
 // ascending boundary id: one thread per cell over the boundaries sorted by
 // (cell, id) at mesh creation.
@@ -54,23 +54,24 @@ __global__ void k_bl_ratearea(const double *__restrict__ flowin, const double *_
 }
 
 // Loop 4 per outlet boundary (MassKernels.ipp:437-451): massFlux from the
-// area rate, the unit normal, the outlet velocities.
+// area rate, the unit normal, the outlet velocities. One thread per outlet
+// boundary (list entry k: its id, its face in the caller's numbering and in
+// the mesh's); the mass fluxes also densely, for their sum.
 template <bool F32>
-__global__ void k_bl4_update(int nB, const int *__restrict__ bndRegion, const int *__restrict__ regionType,
-                             const double *__restrict__ splvl, const int *__restrict__ mapMF,
-                             const int *__restrict__ bndFaceInt, const double4 *__restrict__ fg64,
+__global__ void k_bl4_update(int n, const int *__restrict__ id, const int *__restrict__ face,
+                             const int *__restrict__ faceInt, const int *__restrict__ bndRegion,
+                             const double *__restrict__ splvl, const double4 *__restrict__ fg64,
                              const double4 *__restrict__ fc64, double *__restrict__ massFlux, double *__restrict__ uB,
                              double *__restrict__ vB, double *__restrict__ wB, const double *__restrict__ denB,
-                             const double *__restrict__ ratearea) {
+                             const double *__restrict__ ratearea, double *__restrict__ vals) {
     using O = BndOps<F32>;
-    int ib = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ib >= nB) return;
-    int ir = bndRegion[ib];
-    if (regionType[ir] != CUPCFD_RTYPE_OUTLET) return;
-    int i = mapMF[ib], fi = bndFaceInt[ib];
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int ib = id[k], fi = faceInt[k], ir = bndRegion[ib];
     double area = fc64[fi].w;
     double m = O::mul(O::mul(*ratearea, area), splvl[ir]);
-    massFlux[i] = m;
+    massFlux[face[k]] = m;
+    vals[k] = m;
     double faceFlux = O::div(O::div(m, denB[ib]), area);
     // EuclideanVector::normalise (EuclideanVector.cpp:100-109), length from a
     // dot product accumulated from 0 (EuclideanVector.cpp:83-98)
@@ -93,17 +94,18 @@ __global__ void k_bl4_update(int nB, const int *__restrict__ bndRegion, const in
 // Loop 5 per outlet boundary (MassKernels.ipp:495-508): massFlux scaled by
 // its region's factor, optional velocity scaling.
 template <bool F32>
-__global__ void k_bl5_update(int nB, const int *__restrict__ bndRegion, const int *__restrict__ regionType,
-                             const int *__restrict__ mapMF, double *__restrict__ massFlux,
+__global__ void k_bl5_update(int n, const int *__restrict__ id, const int *__restrict__ face,
+                             const int *__restrict__ bndRegion, double *__restrict__ massFlux,
                              const double *__restrict__ flowFact, double *__restrict__ uB, double *__restrict__ vB,
-                             double *__restrict__ wB, double fact, int solveU, int solveV, int solveW) {
-    int ib = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ib >= nB) return;
-    int ir = bndRegion[ib];
-    if (regionType[ir] != CUPCFD_RTYPE_OUTLET) return;
+                             double *__restrict__ wB, double fact, int solveU, int solveV, int solveW,
+                             double *__restrict__ vals) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
     using O = BndOps<F32>;
-    int i = mapMF[ib];
-    massFlux[i] = O::mul(massFlux[i], flowFact[ir]);
+    const int ib = id[k], i = face[k];
+    const double m = O::mul(massFlux[i], flowFact[bndRegion[ib]]);
+    massFlux[i] = m;
+    vals[k] = m;
     if (solveU) uB[ib] = O::mul(uB[ib], fact);
     if (solveV) vB[ib] = O::mul(vB[ib], fact);
     if (solveW) wB[ib] = O::mul(wB[ib], fact);

@@ -1012,6 +1012,60 @@ __global__ void k_check_regions(int nB, int nR, const int *__restrict__ br, int 
 }
 }  // namespace
 
+namespace {
+
+// faces of listed boundaries
+__global__ void k_list_faces(int n, const int *__restrict__ id, const int *__restrict__ faceRef,
+                             const int *__restrict__ faceInt, int *__restrict__ ref, int *__restrict__ internal) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    ref[k] = faceRef[id[k]];
+    internal[k] = faceInt[id[k]];
+}
+
+// The boundary lists of regions (struct BndLists); every region id is in range.
+int build_bnd_lists(cupcfd_gpu_mesh *m, int nR, const int32_t *type, const int32_t *bndRegion) {
+    BndLists &l = m->bndLists;
+    l.id = l.faceRef = l.faceInt = l.regionPlace = nullptr;
+    for (int &s : l.typeStart) s = 0;
+    const int nB = m->nB;
+    bool any = false;
+    for (int r = 0; r < nR; r++) any |= type[r] != CUPCFD_RTYPE_DEFAULT;
+    if (!any || nB == 0 || !m->bndMapsOk) return CUPCFD_E_SUCCESS;
+    // both lists by counting: a boundary's place is its group's next one
+    std::vector<int> start((size_t) nR + 1, 0), lists(2 * (size_t) nB);
+    int typeStart[6] = {};
+    for (int b = 0; b < nB; b++) start[(size_t) bndRegion[b] + 1]++;
+    for (int r = 0; r < nR; r++) typeStart[type[r] + 1] += start[(size_t) r + 1];
+    for (int r = 0; r < nR; r++) start[(size_t) r + 1] += start[r];
+    for (int t = 0; t < 5; t++) typeStart[t + 1] += typeStart[t];
+    std::vector<int> at(start.begin(), start.end() - 1);
+    int tat[5];
+    std::copy(typeStart, typeStart + 5, tat);
+    for (int b = 0; b < nB; b++) {
+        const int t = type[bndRegion[b]], k = tat[t]++;
+        lists[(size_t) k] = b;
+        lists[(size_t) nB + at[bndRegion[b]]++] = k - typeStart[t];
+    }
+    if (!l.storage) CG_TRY(m->alloc(&l.storage, 4 * (size_t) nB));
+    if (l.regionCap < nR) {
+        CG_TRY(m->alloc(&l.regionStart, (size_t) nR + 1));
+        l.regionCap = nR;
+    }
+    cudaStream_t st = m->stream;
+    int *id = l.storage, *place = id + nB, *ref = place + nB, *internal = ref + nB;
+    CG_CHECK_CUDA(cudaMemcpyAsync(id, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice, st));
+    CG_CHECK_CUDA(cudaMemcpyAsync(l.regionStart, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice, st));
+    k_list_faces<<<grid_for(nB, 256), 256, 0, st>>>(nB, id, m->bndFaceRef, m->bndFaceInt, ref, internal);
+    CG_LAUNCHED();
+    CG_CHECK_CUDA(cudaStreamSynchronize(st));
+    l.id = id; l.faceRef = ref; l.faceInt = internal; l.regionPlace = place;
+    std::copy(typeStart, typeStart + 6, l.typeStart);
+    return CUPCFD_E_SUCCESS;
+}
+
+}  // namespace
+
 extern "C" int cupcfd_gpu_mesh_set_regions(cupcfd_gpu_mesh *m, int32_t nR, const int32_t *type, const double *uvw,
                                            const double *den, const int32_t *bndRegion, int32_t nB) {
     clear_error();
@@ -1048,6 +1102,7 @@ extern "C" int cupcfd_gpu_mesh_set_regions(cupcfd_gpu_mesh *m, int32_t nR, const
         CG_RETURN_IF(h != 0, CUPCFD_E_INVALID_INDEX, "set_regions: a boundary's region id is out of range");
     }
     CG_CHECK_CUDA(cudaStreamSynchronize(st));
+    CG_TRY(build_bnd_lists(m, nR, type, bndRegion));
     m->nR = nR;
     m->hRegionType.assign(type, type + nR);
     m->uvwCarryValid = false;  // the carried-value sources depend on the region types

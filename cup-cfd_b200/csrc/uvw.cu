@@ -20,7 +20,7 @@ namespace {
 
 constexpr int BT = 256;
 // scratch slots of the host-buffer call (kept across calls)
-enum UvwSlot { U_CELLS = 60, U_GRADS, U_VEC, U_TMP, U_MF, U_RF, U_BND, U_BLK, U_SELC, U_SELV, U_SELR, U_SPAN };
+enum UvwSlot { U_CELLS = 60, U_GRADS, U_VEC, U_TMP, U_MF, U_RF, U_BND, U_BLK, U_VALS, U_SPAN };
 
 template <class T>
 int slot(cupcfd_gpu_mesh *m, int s, size_t n, T **p) {
@@ -395,18 +395,14 @@ extern "C" int cupcfd_gpu_dev_uvw_bnds_loop1(cupcfd_gpu_mesh *m, void *stream) {
     if (m->nB > 0) {
         // wall boundaries add their shear onto their region's force tangent
         // in boundary order (UVWKernels.ipp:527-544)
-        int *cnt, *regs;
-        double *vals;
-        CG_TRY(slot(m, U_SELC, (size_t) m->nB / SEL_T + 2, &cnt));
-        CG_TRY(slot(m, U_SELV, 3 * (size_t) m->nB, &vals));
-        CG_TRY(slot(m, U_SELR, (size_t) m->nB, &regs));
         // (in float on a mesh of the reference's T = float instantiation)
-        const SelArgs sa{m->nB, m->bndRegion, m->regionType, CUPCFD_RTYPE_WALL};
+        double *vals;
+        CG_TRY(slot(m, U_VALS, 3 * (size_t) m->nB, &vals));
         const int rc = m->realSize == 4
-                           ? launch_ordered_sum<3, true>(sa, m->bndShear, 3, 0, nullptr, nullptr, 0.0, nullptr,
-                                                         m->regionFT, m->nR, cnt, vals, regs, st)
-                           : launch_ordered_sum<3>(sa, m->bndShear, 3, 0, nullptr, nullptr, 0.0, nullptr, m->regionFT,
-                                                   m->nR, cnt, vals, regs, st);
+                           ? launch_gathered_sum<true>(m, CUPCFD_RTYPE_WALL, m->bndLists.id, m->bndShear, 3, 0, 3, vals,
+                                                       nullptr, m->regionFT, st)
+                           : launch_gathered_sum<false>(m, CUPCFD_RTYPE_WALL, m->bndLists.id, m->bndShear, 3, 0, 3, vals,
+                                                        nullptr, m->regionFT, st);
         CG_TRY(rc);
     }
     return CUPCFD_E_SUCCESS;

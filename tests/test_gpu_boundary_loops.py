@@ -206,3 +206,55 @@ def test_boundary_loop_errors(cg, gpu):
     assert mesh.set_region_split(splvl[:-1]) == cg.E_ARRAY_SIZE_MISMATCH
     rc = cg.lib().cupcfd_gpu_flux_mass_dolfyn_boundary_loop3(mesh.h, 1.0, None)
     assert rc == cg.E_NULL_PTR
+
+
+def _values(kind, n, rng):
+    u, sign = rng.uniform(1e-6, 1e-2, n), rng.choice([-1.0, 1.0], n)
+    return {"one sign": -u, "both signs": u * sign,
+            "ties": rng.integers(-500, 500, n) * 2.0 ** -rng.integers(0, 40, n),   # few bits: halves of a unit
+            "powers": sign * 2.0 ** rng.integers(-30, 30, n),
+            "zeros": np.where(rng.uniform(size=n) < 0.9, 0.0 * sign, u),
+            "tiny": u * 2.0 ** -1060,                                               # subnormal, also as float
+            "huge": np.where(np.arange(n) % 1000 == 700, 1e35, u) * sign,
+            "infinite": np.where(np.arange(n) == n // 2, np.inf, u),
+            "nan": np.where(np.arange(n) == n // 3, np.nan, u)}[kind]
+
+
+@pytest.mark.parametrize("n", [0, 1, 33, 4095, 4096, 4097, 8200])   # a block holds 4,096 additions at a time
+@pytest.mark.parametrize("kind", ["one sign", "both signs", "ties", "powers", "zeros", "tiny", "huge", "infinite", "nan"])
+def test_ordered_sum_rounds_as_the_chain(cg, gpu, kind, n):
+    """Loop 1's and loop 2's sums against the chain of additions itself, in
+    double and in float: values of one sign, values that keep the sum crossing
+    powers of two, ties, zeros of both signs, subnormals, infinities, NaN."""
+    rng = np.random.default_rng(100 + n)
+    mesh = cg.Mesh.structgen(40, 41, 42, order=cg.ORDER_OWNER)
+    nB, nF = mesh.nBoundaries, mesh.nFaces
+    face = np.empty(nB, np.int64)
+    bnd = mesh.geometry()["faceBnd"]
+    face[bnd[bnd >= 0]] = np.nonzero(bnd >= 0)[0]
+    chosen = np.sort(rng.choice(nB, n, replace=False))
+    region = np.zeros(nB, np.int32)
+    vals = _values(kind, n, rng)
+    for rtype in (1, 2):
+        # three regions of the type, interleaved in boundary order
+        region[chosen] = 1 + np.arange(n) % 3
+        assert mesh.set_regions([0, rtype, rtype, rtype], np.zeros((4, 3)), np.ones(4), region) == cg.E_SUCCESS
+        for t in (np.float64, np.float32):
+            mf = np.zeros(nF, t)
+            with np.errstate(over="ignore", invalid="ignore", under="ignore"):
+                v = vals.astype(t)
+                mf[face[chosen]] = v
+                total, acc = t(0), np.array([0.5, 0.25, -3.0, 0.0], t)
+                want_acc = acc.copy()
+                for k in range(n):
+                    total = total + v[k]
+                    want_acc[1 + k % 3] += v[k]
+            if rtype == 1:
+                rc, got = cg.FluxMassDolfynBoundaryLoop1(mesh, mf)
+            else:
+                rc, got = cg.FluxMassDolfynBoundaryLoop2(mesh, mf, acc)
+            assert rc == cg.E_SUCCESS, cg.last_error()
+            same = lambda a, b: np.array_equal(np.asarray(a, np.float64), np.asarray(b, np.float64), equal_nan=True)
+            assert same(got, total), (t, got, total)
+            if rtype == 2:
+                assert same(acc, want_acc), (t, acc, want_acc)
