@@ -67,14 +67,14 @@ inline SellView sell(const cupcfd_gpu_mesh *m) {
 // -6 when those lists also have their run form (struct Sell), else 0 (the
 // general kernels).
 inline int list_form(const cupcfd_gpu_mesh *m) { return m->fullWidth == 6 && m->sell.runs ? -6 : m->fullWidth; }
-// launches the L2-prefetch kernel template K for the mesh's list form
-#define CG_LAUNCH_PF_BLOCK(m, K, grid, block, st, ...)                          \
-    do {                                                                        \
-        if (list_form(m) == -6) K<-6><<<(grid), (block), 0, (st)>>>(__VA_ARGS__); \
-        else if (list_form(m) == 6) K<6><<<(grid), (block), 0, (st)>>>(__VA_ARGS__); \
-        else K<0><<<(grid), (block), 0, (st)>>>(__VA_ARGS__);                   \
+// launches the L2-prefetch kernel template K over the mesh's tiles, for its
+// list form, in blocks of BLOCK<form> threads
+#define CG_LAUNCH_PF(m, K, BLOCK, st, ...)                                                                           \
+    do {                                                                                                             \
+        if (list_form(m) == -6) K<-6><<<m->nTiles * (TILE_CELLS / BLOCK<-6>), BLOCK<-6>, 0, (st)>>>(__VA_ARGS__);    \
+        else if (list_form(m) == 6) K<6><<<m->nTiles * (TILE_CELLS / BLOCK<6>), BLOCK<6>, 0, (st)>>>(__VA_ARGS__);   \
+        else K<0><<<m->nTiles * (TILE_CELLS / BLOCK<0>), BLOCK<0>, 0, (st)>>>(__VA_ARGS__);                          \
     } while (0)
-#define CG_LAUNCH_PF(m, K, grid, st, ...) CG_LAUNCH_PF_BLOCK(m, K, grid, BLK, st, __VA_ARGS__)
 
 // ---------------------------------------------------------------------------
 // device timers (cupcfd_gpu_timing_*): a KTIMER scope records one event
@@ -175,10 +175,10 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
 #undef PF_KERNEL
     static_assert(sizeof(pfKern) / sizeof(pfKern[0]) == PF_COUNT, "one kernel per PfKernel");
     static_assert(PF_COUNT <= (int) (sizeof(m->prefetchWave) / sizeof(m->prefetchWave[0])), "room for every wave");
-    // block sizes: 64 threads (TileBlock) for the forward kernels and the
-    // FP32 adjoint, 256 (one tile) for the FP64 adjoint and the adjoint parts
-    const int pfBlock[PF_COUNT] = {CUPCFD_FWD_BLOCK,      CUPCFD_FWD_BLOCK, CUPCFD_FWD_BLOCK, TILE_CELLS,
-                                   CUPCFD_FWD_MADJ_BLOCK, CUPCFD_GADJ_BLOCK, TILE_CELLS};
+#define PF_BLOCK(B) (wf == -6 ? B<-6> : wf == 6 ? B<6> : B<0>)
+    const int pfBlock[PF_COUNT] = {PF_BLOCK(PF_BLOCK_FWD),      PF_BLOCK(PF_BLOCK_ADJ),  PF_BLOCK(PF_BLOCK_FWD_F64), PF_BLOCK(PF_BLOCK_ADJ_F64),
+                                   PF_BLOCK(PF_BLOCK_FWD_MADJ), PF_BLOCK(PF_BLOCK_GADJ), PF_BLOCK(PF_BLOCK_MADJ)};
+#undef PF_BLOCK
     // prefetch distance in waves, in quarters, measured at 256^3 (same box):
     // 1.25 waves for the forward+mass adjoint (0.538 ms against 0.546 at 1
     // wave, 0.541 at 1.5, 0.581 at 0.75), the separate FP32 forward and
@@ -293,6 +293,9 @@ int mesh_post_build(cupcfd_gpu_mesh *m, cudaStream_t st) {
     CG_LAUNCHED();
     CG_CHECK_CUDA(cudaMemcpyAsync(&m->bandwidth, bw, sizeof(int), cudaMemcpyDeviceToHost, st));
     CG_TRY(tiles_setup(m, st));
+    // the forward calls' loss partials (one per warp), so that no call stops to allocate them
+    double *part;
+    CG_TRY(scratch(m, S_LOSS, (size_t) grid_for(nC, BLK) * (TILE_CELLS / 32), &part));
     CG_CHECK_CUDA(cudaStreamSynchronize(st));
     return CUPCFD_E_SUCCESS;
 }
@@ -448,8 +451,7 @@ const char *launch_fwd_f32(const cupcfd_gpu_mesh *m, const void *phi, const void
                            int *group) {
     *group = 1;
     if (m->tiles && aligned16(phi) && aligned16(state) && (!gface || aligned16(gface))) {
-        CG_LAUNCH_PF_BLOCK(m, k_fwd_f32_pf, grid_for(m->nC, BLK) * (TILE_CELLS / CUPCFD_FWD_BLOCK), CUPCFD_FWD_BLOCK,
-                           st, m->nC, sell(m), m->fg32, (const float *) phi, (const float *) phiB, m->vol,
+        CG_LAUNCH_PF(m, k_fwd_f32_pf, PF_BLOCK_FWD, st, m->nC, sell(m), m->fg32, (const float *) phi, (const float *) phiB, m->vol,
                            (const float4 *) state, (const float *) gface, (float *) grad, (float *) massFlux, part,
                            m->nC, prefetch_args(m, PF_FWD_F32));
         *group = TILE_CELLS / 32;
@@ -463,16 +465,13 @@ const char *launch_fwd_f32(const cupcfd_gpu_mesh *m, const void *phi, const void
 }
 
 // FP64 forward: the L2-prefetch kernel when the tile ranges exist and the
-// arrays allow whole 16-byte ranges (state blocks of an even cell count),
-// else the plain one. Identical results.
+// arrays start on 16-byte boundaries, else the plain one. Identical results.
 const char *launch_fwd_f64(const cupcfd_gpu_mesh *m, const void *phi, const void *phiB, const void *state,
                            const void *gface, void *grad, void *massFlux, double *part, cudaStream_t st,
                            int *group) {
     *group = 1;
-    if (m->tiles && aligned16(phi) && aligned16(state) && (!gface || aligned16(gface)) &&
-        m->nC % 2 == 0) {
-        CG_LAUNCH_PF_BLOCK(m, k_fwd_f64_pf, grid_for(m->nC, BLK) * (TILE_CELLS / CUPCFD_FWD_BLOCK), CUPCFD_FWD_BLOCK,
-                           st, m->nC, sell(m), m->fg64, (const double *) phi, (const double *) phiB, m->vol,
+    if (m->tiles && aligned16(phi) && aligned16(state) && (!gface || aligned16(gface))) {
+        CG_LAUNCH_PF(m, k_fwd_f64_pf, PF_BLOCK_FWD_F64, st, m->nC, sell(m), m->fg64, (const double *) phi, (const double *) phiB, m->vol,
                            (const double *) state, (const double *) gface, (double *) grad, (double *) massFlux,
                            part, m->nC, prefetch_args(m, PF_FWD_F64));
         *group = TILE_CELLS / 32;
@@ -534,18 +533,18 @@ extern "C" int cupcfd_gpu_dev_adjoint(cupcfd_gpu_mesh *m, int32_t precision, con
     unsigned grid = grid_for(m->nC, BLK);
     KernelTimer kt(nullptr, st);
     if (precision == CUPCFD_PREC_F64 && m->tiles && aligned16(grad) && aligned16(state) &&
-        aligned16(gface) && m->nC % 2 == 0) {
+        aligned16(gface)) {
         kt.set_name("k_adj_f64_pf");
-        CG_LAUNCH_PF(m, k_adj_f64_pf, grid, st, m->nC, sell(m), m->fg64, (const double *) grad, 2.0,
+        CG_LAUNCH_PF(m, k_adj_f64_pf, PF_BLOCK_ADJ_F64, st, m->nC, sell(m), m->fg64, (const double *) grad, 2.0,
                      (const double *) state, (const double *) gface, (double *) phiBar, (double *) phiBBar,
                      (double *) stateBar, m->nC, prefetch_args(m, PF_ADJ_F64));
     } else if (precision == CUPCFD_PREC_F64) {
         kt.set_name("k_adj_f64");
         k_adj_f64<<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, (const double *) grad, 2.0, (const double *) state,
                                         (const double *) gface, (double *) phiBar, (double *) phiBBar, (double *) stateBar, m->nC);
-    } else if (m->tiles && aligned16(grad) && aligned16(state) && aligned16(gface) && m->nC % 4 == 0) {
+    } else if (m->tiles && aligned16(grad) && aligned16(state) && aligned16(gface)) {
         kt.set_name("k_adj_f32_pf");
-        CG_LAUNCH_PF_BLOCK(m, k_adj_f32_pf, grid * (TILE_CELLS / CUPCFD_FWD_BLOCK), CUPCFD_FWD_BLOCK, st, m->nC,
+        CG_LAUNCH_PF(m, k_adj_f32_pf, PF_BLOCK_ADJ, st, m->nC,
                            sell(m), m->fg32, (const float *) grad, 2.f, (const float4 *) state, (const float *) gface,
                            (float *) phiBar, (float *) phiBBar, (float4 *) stateBar, m->nC,
                            prefetch_args(m, PF_ADJ_F32));
@@ -558,6 +557,14 @@ extern "C" int cupcfd_gpu_dev_adjoint(cupcfd_gpu_mesh *m, int32_t precision, con
     return CUPCFD_E_SUCCESS;
 }
 
+namespace {
+// Above this many tiles the loss reduction runs on the mesh's second stream,
+// beside the gradient adjoint; below, the events that tie the streams cost
+// more than the reduction itself: 14.4 us a call against 16.3 at 128 tiles
+// (32^3 cells), 18.6 against 15.1 at 432 (48^3).
+constexpr unsigned LOSS_BESIDE_TILES = 148;
+}  // namespace
+
 extern "C" int cupcfd_gpu_dev_forward_adjoint(cupcfd_gpu_mesh *m, int32_t precision, const void *phi, const void *phiB,
                                               const void *state, const void *gface, void *grad, void *massFlux,
                                               void *phiBar, void *phiBBar, void *stateBar, double *loss, void *stream) {
@@ -567,7 +574,7 @@ extern "C" int cupcfd_gpu_dev_forward_adjoint(cupcfd_gpu_mesh *m, int32_t precis
     if (!lp) CG_TRY(scratch(m, S_NORM, 1, &lp));
     CG_TRY(check_prec(m, precision));
     if (precision == CUPCFD_PREC_F32C && m->tiles && aligned16(phi) && aligned16(state) &&
-        aligned16(gface) && aligned16(grad) && aligned16(stateBar) && m->nC % 4 == 0) {
+        aligned16(gface) && aligned16(grad) && aligned16(stateBar)) {
         // forward with the mass-flux adjoint, then the gradient adjoint: the
         // state and gface stream through one pass only
         CG_RETURN_IF(!phi || !state || !grad || !massFlux || !phiBar || !stateBar || (m->nB > 0 && (!phiB || !phiBBar)),
@@ -584,31 +591,34 @@ extern "C" int cupcfd_gpu_dev_forward_adjoint(cupcfd_gpu_mesh *m, int32_t precis
         PrefetchArgs pf = prefetch_args(m, PF_FWD_MADJ), pfg = prefetch_args(m, PF_GADJ);
         {
             KTIMER("k_fwd_madj_f32_pf", st);
-            CG_LAUNCH_PF_BLOCK(m, k_fwd_madj_f32_pf, grid * (TILE_CELLS / CUPCFD_FWD_MADJ_BLOCK), CUPCFD_FWD_MADJ_BLOCK,
-                         st, m->nC, sell(m), m->fg32, (const float *) phi,
+            CG_LAUNCH_PF(m, k_fwd_madj_f32_pf, PF_BLOCK_FWD_MADJ, st, m->nC, sell(m), m->fg32, (const float *) phi,
                          (const float *) phiB, m->vol, (const float4 *) state, (const float *) gface, (float *) grad,
                          (float *) massFlux, (float4 *) stateBar, part, m->nC, pf);
             CG_LAUNCHED();
         }
-        {
-            // the FP64 loss reduction (one block) runs on the mesh's second
-            // stream beside the gradient adjoint, which does not need it;
-            // the caller's stream waits for both
-            cudaStream_t so = m->outStream;
+        // the FP64 loss reduction (one block) runs on the mesh's second stream
+        // beside the gradient adjoint, which does not need it; the caller's
+        // stream waits for both
+        const bool beside = grid > LOSS_BESIDE_TILES;
+        cudaStream_t so = st;
+        if (beside) {
+            so = m->outStream;
             CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[0], st));
             CG_CHECK_CUDA(cudaStreamWaitEvent(so, m->pipeEv[0], 0));
+        }
+        {
             KTIMER("k_reduce_partials", so);
             k_reduce_partials<WPT><<<1, 1024, 0, so>>>((int) grid, part, lp);
             CG_LAUNCHED();
         }
-        CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[1], m->outStream));
+        if (beside) CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[1], so));
         {
             KTIMER("k_gadj_f32_pf", st);
-            CG_LAUNCH_PF_BLOCK(m, k_gadj_f32_pf, grid * (TILE_CELLS / CUPCFD_GADJ_BLOCK), CUPCFD_GADJ_BLOCK, st, m->nC, sell(m), m->fg32, (const float *) grad, 2.f,
+            CG_LAUNCH_PF(m, k_gadj_f32_pf, PF_BLOCK_GADJ, st, m->nC, sell(m), m->fg32, (const float *) grad, 2.f,
                          (float *) phiBar, (float *) phiBBar, m->nC, pfg);
             CG_LAUNCHED();
         }
-        CG_CHECK_CUDA(cudaStreamWaitEvent(st, m->pipeEv[1], 0));
+        if (beside) CG_CHECK_CUDA(cudaStreamWaitEvent(st, m->pipeEv[1], 0));
         return CUPCFD_E_SUCCESS;
     }
     CG_TRY(cupcfd_gpu_dev_forward(m, precision, phi, phiB, state, gface, grad, massFlux, lp, stream));
@@ -960,10 +970,10 @@ int launch_adj_part(const cupcfd_gpu_mesh *m, bool f64, const void *g, double hs
         (gradPart ? hscale == 2.0 && aligned16(g) : hscale == 0.0 && !g && aligned16(state) && aligned16(gface))) {
         kt.set_name(gradPart ? "k_gadj_f32_pf" : "k_madj_f32_pf");
         if (gradPart)
-            CG_LAUNCH_PF_BLOCK(m, k_gadj_f32_pf, grid * (TILE_CELLS / CUPCFD_GADJ_BLOCK), CUPCFD_GADJ_BLOCK, st, m->nC, sell(m), m->fg32, (const float *) g, 2.f,
+            CG_LAUNCH_PF(m, k_gadj_f32_pf, PF_BLOCK_GADJ, st, m->nC, sell(m), m->fg32, (const float *) g, 2.f,
                          (float *) phiBar, (float *) phiBBar, m->nC, prefetch_args(m, PF_GADJ));
         else
-            CG_LAUNCH_PF(m, k_madj_f32_pf, grid, st, m->nC, sell(m), m->fg32, (const float4 *) state,
+            CG_LAUNCH_PF(m, k_madj_f32_pf, PF_BLOCK_MADJ, st, m->nC, sell(m), m->fg32, (const float4 *) state,
                          (const float *) gface, (float4 *) stateBar, m->nC, prefetch_args(m, PF_MADJ));
         CG_LAUNCHED();
         return CUPCFD_E_SUCCESS;

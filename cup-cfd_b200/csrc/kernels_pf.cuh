@@ -13,6 +13,18 @@
 
 namespace cupcfd_gpu {
 
+// Threads per block of each kernel, by list form. Measured on full lists: the
+// FP32 step on a permuted 192^3 mesh 431 us in 64-thread blocks (gradient
+// adjoint in 256), 425 in 128, 431 in 256, 464 in 512; FP64 forward and
+// adjoint at 96^3 70 / 92 in 64, 72 / 87 in 128, 74 / 90 in 256.
+template <int WF> constexpr int PF_BLOCK_FWD = 64;
+template <int WF> constexpr int PF_BLOCK_ADJ = 64;
+template <int WF> constexpr int PF_BLOCK_FWD_F64 = 64;
+template <int WF> constexpr int PF_BLOCK_ADJ_F64 = 128;
+template <int WF> constexpr int PF_BLOCK_FWD_MADJ = WF == -6 ? 64 : 128;
+template <int WF> constexpr int PF_BLOCK_GADJ = WF == -6 ? 64 : 128;
+template <int WF> constexpr int PF_BLOCK_MADJ = 256;
+
 // ---------------------------------------------------------------------------
 // L2 prefetch variant: the unstaged one-cell-per-thread kernels (the same
 // per-cell bodies, so bit-identical results), where one lane per 256-cell
@@ -27,24 +39,20 @@ namespace cupcfd_gpu {
 // same order, so the same bits).
 // ---------------------------------------------------------------------------
 
-// The separate forward and FP32 adjoint kernels run in blocks of
-// CUPCFD_FWD_BLOCK = 64 threads (TileBlock), the forwards with one loss
+// The separate forward and FP32 adjoint kernels run in blocks of 64 threads
+// (TileBlock), the forwards with one loss
 // partial per warp, folded per tile by k_group_partials before the fixed-
 // order sum. At 256^3 on one box: FP32 forward 0.477-0.485 ms against
 // 0.503-0.533 in 256-thread blocks, FP32 adjoint 0.518-0.529 against
-// 0.543-0.583, FP64 forward 0.698-0.704 against 0.707-0.717. The FP64
-// adjoint keeps 256-thread blocks (slower in 64: 0.835 against 0.81 ms).
-#ifndef CUPCFD_FWD_BLOCK
-#define CUPCFD_FWD_BLOCK 64
-#endif
+// 0.543-0.583, FP64 forward 0.698-0.704 against 0.707-0.717.
 template <int WF>
-__global__ void __launch_bounds__(CUPCFD_FWD_BLOCK, CUPCFD_MINB_F32 *TILE_CELLS / CUPCFD_FWD_BLOCK)
+__global__ void __launch_bounds__(PF_BLOCK_FWD<WF>, CUPCFD_MINB_F32 *TILE_CELLS / PF_BLOCK_FWD<WF>)
     k_fwd_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ phi,
                  const float *__restrict__ phiB, const double *__restrict__ vol, const float4 *__restrict__ st,
                  const float *__restrict__ gface, float *__restrict__ g, float *__restrict__ mflux,
                  double *__restrict__ lossPart, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    const TileBlock<CUPCFD_FWD_BLOCK> tb(pf);
+    const TileBlock<PF_BLOCK_FWD<WF>> tb(pf);
     const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[3] = {phi, st, vol};
@@ -53,16 +61,16 @@ __global__ void __launch_bounds__(CUPCFD_FWD_BLOCK, CUPCFD_MINB_F32 *TILE_CELLS 
     double l = 0.0;
     if (c < nC) l = fwd_cell_f32<CUPCFD_FWD_CHUNK, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, ldc);
     if (tb.lead) prefetch_tile<3>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
-    if (lossPart) warp_partial_store<CUPCFD_FWD_BLOCK>(l, c, lossPart);
+    if (lossPart) warp_partial_store<PF_BLOCK_FWD<WF>>(l, c, lossPart);
 }
 
 template <int WF>
-__global__ void __launch_bounds__(CUPCFD_FWD_BLOCK, CUPCFD_MINB_F32 *TILE_CELLS / CUPCFD_FWD_BLOCK)
+__global__ void __launch_bounds__(PF_BLOCK_ADJ<WF>, CUPCFD_MINB_F32 *TILE_CELLS / PF_BLOCK_ADJ<WF>)
     k_adj_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ g, float hscale,
                  const float4 *__restrict__ st, const float *__restrict__ gface, float *__restrict__ phibar,
                  float *__restrict__ phibBar, float4 *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    const TileBlock<CUPCFD_FWD_BLOCK> tb(pf);
+    const TileBlock<PF_BLOCK_ADJ<WF>> tb(pf);
     const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[4] = {g, g + ldc, g + 2 * ldc, st};
@@ -75,13 +83,13 @@ __global__ void __launch_bounds__(CUPCFD_FWD_BLOCK, CUPCFD_MINB_F32 *TILE_CELLS 
 // FP64 forward (fwd_cell_f64, exact reference arithmetic) with the same L2
 // prefetch; the state's four component blocks are prefetched one by one.
 template <int WF>
-__global__ void __launch_bounds__(CUPCFD_FWD_BLOCK, CUPCFD_MINB_FWD_F64 *TILE_CELLS / CUPCFD_FWD_BLOCK)
+__global__ void __launch_bounds__(PF_BLOCK_FWD_F64<WF>, CUPCFD_MINB_FWD_F64 *TILE_CELLS / PF_BLOCK_FWD_F64<WF>)
     k_fwd_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ phi,
                  const double *__restrict__ phiB, const double *__restrict__ vol, const double *__restrict__ st,
                  const double *__restrict__ gface, double *__restrict__ g, double *__restrict__ mflux,
                  double *__restrict__ lossPart, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    const TileBlock<CUPCFD_FWD_BLOCK> tb(pf);
+    const TileBlock<PF_BLOCK_FWD_F64<WF>> tb(pf);
     const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[6] = {phi, vol, st, st + ldc, st + 2 * ldc, st + 3 * ldc};
@@ -90,35 +98,34 @@ __global__ void __launch_bounds__(CUPCFD_FWD_BLOCK, CUPCFD_MINB_FWD_F64 *TILE_CE
     double l = 0.0;
     if (c < nC) l = fwd_cell_f64<CUPCFD_FWD_CHUNK_F64, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, ldc);
     if (tb.lead) prefetch_tile<6>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
-    if (lossPart) warp_partial_store<CUPCFD_FWD_BLOCK>(l, c, lossPart);
+    if (lossPart) warp_partial_store<PF_BLOCK_FWD_F64<WF>>(l, c, lossPart);
 }
 
 // FP64 adjoint (adj_cell_f64) with the same L2 prefetch.
 template <int WF>
-__global__ void __launch_bounds__(TILE_CELLS, CUPCFD_MINB_ADJ_F64)
+__global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, CUPCFD_MINB_ADJ_F64 *TILE_CELLS / PF_BLOCK_ADJ_F64<WF>)
     k_adj_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ g, double hscale,
                  const double *__restrict__ st, const double *__restrict__ gface, double *__restrict__ phibar,
                  double *__restrict__ phibBar, double *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    int c = blockIdx.x * T + threadIdx.x;
-    const int tp = blockIdx.x + pf.dist;
-    const bool lead = threadIdx.x == T - 32 && tp < pf.nTiles;
+    const TileBlock<PF_BLOCK_ADJ_F64<WF>> tb(pf);
+    const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[7] = {g, g + ldc, g + 2 * ldc, st, st + ldc, st + 2 * ldc, st + 3 * ldc};
     const int cellBytes[7] = {T * 8, T * 8, T * 8, T * 8, T * 8, T * 8, T * 8};
-    if (lead) fetch_ranges_async(&s_rng, pf.desc + tp);
+    if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     if (c < nC) adj_cell_f64<false, CUPCFD_ADJ_CHUNK_F64, WF>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
-    if (lead) prefetch_tile<7>(pf, tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
+    if (tb.lead) prefetch_tile<7>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
 }
 
 // Forward with the mass-flux adjoint (fwd_madj_cell_f32), L2 prefetch as
 // k_fwd_f32_pf. With k_gadj_f32_pf it forms the two-launch forward+adjoint:
 // the state and gface are then read by one pass only.
 //
-// It runs in blocks of CUPCFD_FWD_MADJ_BLOCK = 64 threads, four per tile, at
+// It runs in blocks of PF_BLOCK_FWD_MADJ threads, several per tile, at
 // the same registers and warps per SM as 256-thread blocks: a block's slot
 // frees when its two warps end instead of its slowest of eight (measured at
-// 256^3: 0.543 ms against 0.568 ms; 32-thread blocks 0.540). The last block
+// 256^3, 64 threads: 0.543 ms against 0.568 ms; 32-thread blocks 0.540). The last block
 // of a tile prefetches for the tile. The loss partials are one per warp,
 // warp k of tile t at lossPart[k nTiles + t]; k_reduce_partials<8> sums each
 // tile's eight in order, which gives the per-tile value of
@@ -138,17 +145,14 @@ __global__ void __launch_bounds__(TILE_CELLS, CUPCFD_MINB_ADJ_F64)
 #ifndef CUPCFD_MINB_FWD_MADJ
 #define CUPCFD_MINB_FWD_MADJ 4  // in 256-cell tiles per SM
 #endif
-#ifndef CUPCFD_FWD_MADJ_BLOCK
-#define CUPCFD_FWD_MADJ_BLOCK 64
-#endif
 template <int WF>
-__global__ void __launch_bounds__(CUPCFD_FWD_MADJ_BLOCK, CUPCFD_MINB_FWD_MADJ *TILE_CELLS / CUPCFD_FWD_MADJ_BLOCK)
+__global__ void __launch_bounds__(PF_BLOCK_FWD_MADJ<WF>, CUPCFD_MINB_FWD_MADJ *TILE_CELLS / PF_BLOCK_FWD_MADJ<WF>)
     k_fwd_madj_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ phi,
                       const float *__restrict__ phiB, const double *__restrict__ vol, const float4 *__restrict__ st,
                       const float *__restrict__ gface, float *__restrict__ g, float *__restrict__ mflux,
                       float4 *__restrict__ stbar, double *__restrict__ lossPart, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    const TileBlock<CUPCFD_FWD_MADJ_BLOCK> tb(pf);
+    const TileBlock<PF_BLOCK_FWD_MADJ<WF>> tb(pf);
     const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[3] = {phi, st, vol};
@@ -157,7 +161,7 @@ __global__ void __launch_bounds__(CUPCFD_FWD_MADJ_BLOCK, CUPCFD_MINB_FWD_MADJ *T
     double l = 0.0;
     if (c < nC) {
         if constexpr (WF == -6) {
-            __shared__ FwdMadjStage<CUPCFD_FWD_MADJ_BLOCK> stage;
+            __shared__ FwdMadjStage<PF_BLOCK_FWD_MADJ<WF>> stage;
             const CellList<WF> e(sv, c);
             l = e.alternating == 2   ? fwd_madj_cell_staged<2>(c, e, stage, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc)
                 : e.alternating == 1 ? fwd_madj_cell_staged<1>(c, e, stage, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc)
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(CUPCFD_FWD_MADJ_BLOCK, CUPCFD_MINB_FWD_MADJ *T
             l = fwd_madj_cell_f32<CUPCFD_FWD_MADJ_CHUNK, 0, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, stbar, ldc);
     }
     if (tb.lead) prefetch_tile<3>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
-    if (lossPart) warp_partial_store<CUPCFD_FWD_MADJ_BLOCK>(l, c, lossPart);
+    if (lossPart) warp_partial_store<PF_BLOCK_FWD_MADJ<WF>>(l, c, lossPart);
 }
 
 // Gradient part of the adjoint only (adj_cell_f32 without the mass part):
@@ -183,15 +187,12 @@ __global__ void __launch_bounds__(CUPCFD_FWD_MADJ_BLOCK, CUPCFD_MINB_FWD_MADJ *T
 #ifndef CUPCFD_MINB_GADJ
 #define CUPCFD_MINB_GADJ 6
 #endif
-#ifndef CUPCFD_GADJ_BLOCK
-#define CUPCFD_GADJ_BLOCK 64
-#endif
 template <int WF>
-__global__ void __launch_bounds__(CUPCFD_GADJ_BLOCK, CUPCFD_MINB_GADJ *TILE_CELLS / CUPCFD_GADJ_BLOCK)
+__global__ void __launch_bounds__(PF_BLOCK_GADJ<WF>, CUPCFD_MINB_GADJ *TILE_CELLS / PF_BLOCK_GADJ<WF>)
     k_gadj_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ g, float hscale,
                   float *__restrict__ phibar, float *__restrict__ phibBar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    const TileBlock<CUPCFD_GADJ_BLOCK> tb(pf);
+    const TileBlock<PF_BLOCK_GADJ<WF>> tb(pf);
     const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[3] = {g, g + ldc, g + 2 * ldc};
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(CUPCFD_GADJ_BLOCK, CUPCFD_MINB_GADJ *TILE_CELL
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     if (c < nC) {
         if constexpr (WF == -6) {
-            __shared__ GadjStage<CUPCFD_GADJ_BLOCK> stage;
+            __shared__ GadjStage<PF_BLOCK_GADJ<WF>> stage;
             const CellList<WF> e(sv, c);
             if (e.alternating == 2) gadj_cell_staged<2>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
             else if (e.alternating == 1) gadj_cell_staged<1>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
@@ -216,20 +217,19 @@ __global__ void __launch_bounds__(CUPCFD_GADJ_BLOCK, CUPCFD_MINB_GADJ *TILE_CELL
 // host forward+adjoint call runs it once gface is in; with k_gadj_f32_pf for
 // the gradient part it forms the same sums as k_adj_f32_pf, so the same bits.
 template <int WF>
-__global__ void __launch_bounds__(TILE_CELLS, CUPCFD_MINB_F32)
+__global__ void __launch_bounds__(PF_BLOCK_MADJ<WF>, CUPCFD_MINB_F32 *TILE_CELLS / PF_BLOCK_MADJ<WF>)
     k_madj_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float4 *__restrict__ st,
                   const float *__restrict__ gface, float4 *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
-    int c = blockIdx.x * T + threadIdx.x;
-    const int tp = blockIdx.x + pf.dist;
-    const bool lead = threadIdx.x == T - 32 && tp < pf.nTiles;
+    const TileBlock<PF_BLOCK_MADJ<WF>> tb(pf);
+    const int c = tb.c;
     __shared__ int4 s_rng;
     const void *const cellSrc[1] = {st};
     const int cellBytes[1] = {T * 16};
-    if (lead) fetch_ranges_async(&s_rng, pf.desc + tp);
+    if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     if (c < nC)
         adj_cell_f32<false, CUPCFD_ADJ_CHUNK, 0, WF>(c, sv, fg, nullptr, 0.f, st, gface, nullptr, nullptr, stbar, ldc);
-    if (lead) prefetch_tile<1>(pf, tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
+    if (tb.lead) prefetch_tile<1>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
 }
 
 // Largest |c - neighbour| over the incidence lists (the numbering's bandwidth).

@@ -53,11 +53,10 @@ __device__ __forceinline__ int4 ranges_ready(const int4 *src) {
     return *src;
 }
 
-// Blocks smaller than a tile: TILE_CELLS / B blocks of B threads per tile,
-// at the registers and warps per SM of 256-thread blocks. A block's slot
-// frees when its own warps end instead of the slowest of eight. The last
-// block of a tile prefetches for the tile (the lead lane: its last warp's
-// first lane).
+// A kernel's blocks of B threads, one cell a thread, TILE_CELLS / B per tile:
+// a small block's slot frees when its own warps end instead of the slowest of
+// eight. The last block of a tile prefetches for the tile (the lead lane: its
+// last warp's first lane).
 template <int B>
 struct TileBlock {
     static_assert(TILE_CELLS % B == 0 && B % 32 == 0, "whole warps, whole tiles");
@@ -100,9 +99,12 @@ __device__ __forceinline__ void prefetch_tile(const PrefetchArgs &p, int t, cons
         if (gfB > p.nF) gfB = fe & ~(PER16 - 1);
         if (gfB > gfA) bulk_prefetch_l2(gface + gfA, (unsigned) (gfB - gfA) * (unsigned) sizeof(TG));
     }
+    // A component block of an odd cell count starts off a 16-byte boundary:
+    // its range is moved down to one (t >= 1, so it stays in the array).
     if ((long long) (t + 1) * TILE_CELLS <= (long long) p.nC)
         for (int i = 0; i < NCELL; i++)
-            bulk_prefetch_l2(static_cast<const unsigned char *>(cellSrc[i]) + (size_t) t * cellBytes[i],
+            bulk_prefetch_l2(reinterpret_cast<const void *>(
+                                 (reinterpret_cast<uintptr_t>(cellSrc[i]) + (size_t) t * cellBytes[i]) & ~(uintptr_t) 15),
                              (unsigned) cellBytes[i]);
 }
 

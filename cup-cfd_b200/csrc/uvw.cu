@@ -137,7 +137,7 @@ int run_face_loop(cupcfd_gpu_mesh *m, T gammaBlend, T small, const T *u, const T
     auto a16 = [](const void *p) { return ((uintptr_t) p & 15u) == 0; };
     const bool pfOk = m->tiles && m->tileDesc && a16(u) && a16(v) && a16(w) && a16(visC) &&
                       a16(su) && a16(sv) && a16(sw) && a16(au) && a16(av) && a16(aw) && a16(grads) &&
-                      (ldg * (int64_t) sizeof(T)) % 16 == 0 && a16(massFlux) && !prefetch_disabled();
+                      a16(massFlux) && !prefetch_disabled();
     if (pfOk) {
         PrefetchArgs pf;
         pf.desc = (const TileDesc *) m->tileDesc;

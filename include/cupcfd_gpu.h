@@ -467,10 +467,9 @@ int cupcfd_gpu_flux_mass_dolfyn_region_loop_f32(cupcfd_gpu_mesh *mesh, float *fl
  * stream: a cudaStream_t (NULL = the legacy default stream).
  * Every array is aligned to its element (the F32C state to 16 bytes);
  * misaligned pointers are rejected with CUPCFD_E_CONFIG_INVALID_VALUE.
- * F32C forward/adjoint calls whose arrays start on 16-byte boundaries (and,
- * for the adjoint, nCells a multiple of 4) run the staged kernels, which
- * fetch each 256-cell tile's contiguous ranges into shared memory with bulk
- * async copies; other pointers take the unstaged kernels. Results are
+ * Forward/adjoint calls whose arrays start on 16-byte boundaries run the
+ * L2-prefetch kernels, which ask for each 256-cell tile's contiguous ranges a
+ * wave of blocks ahead; other pointers take the plain kernels. Results are
  * bit-identical either way. */
 
 /* Reorders n-component cell data (component blocks of nCells, element type

@@ -333,3 +333,29 @@ def test_irregular_numbering_has_no_run_form(cg, gpu, monkeypatch):
     lists = cg.Mesh.jittered(20, 18, 16, order=cg.ORDER_OWNER)
     monkeypatch.delenv("CUPCFD_RUNS")
     assert cg.Mesh.jittered(20, 18, 16, order=cg.ORDER_OWNER).deviceBytes == lists.deviceBytes
+
+
+@pytest.mark.parametrize("kind,dims,order", [("structgen", (33, 17, 9), "ORDER_OWNER"),     # 5,049 cells: 1 past a multiple of 4
+                                             ("structgen", (37, 7, 10), "ORDER_MORTON"),    # 2,590: 2 past
+                                             ("jittered", (15, 13, 11), "ORDER_RCM"),       # 2,145: 1 past
+                                             ("structgen", (5, 5, 11), "ORDER_OWNER")])     # 275: 3 past, one whole tile
+def test_any_cell_count_takes_the_prefetch_kernels(cg, gpu, kind, dims, order):
+    """Component blocks of a cell count that is no multiple of four start off
+    16-byte boundaries; the L2-prefetch kernels run all the same, with the
+    plain kernels' bits, and the pipeline as two launches."""
+    import torch
+    mesh = _mesh(cg, kind, dims, order)
+    assert mesh.nCells % 4
+    fields = _fields(torch, mesh, 23)
+    a = _run(cg, torch, mesh, *fields, offset=False)
+    assert {"k_fwd_f32_pf", "k_adj_f32_pf"} <= _run.kernels
+    b = _run(cg, torch, mesh, *fields, offset=True)
+    assert {"k_fwd_f32", "k_adj_f32"} <= _run.kernels
+    _assert_same(a, b)
+    cg.timing_read()
+    cg.timing_enable(True)
+    try:
+        _assert_same(_run_pipeline(cg, torch, mesh, *fields, offset=False), b)
+        assert {"k_fwd_madj_f32_pf", "k_gadj_f32_pf"} <= set(cg.timing_read())
+    finally:
+        cg.timing_enable(False)
