@@ -18,7 +18,10 @@ namespace {
 constexpr int BLK = 256;
 
 // the L2-prefetch kernels, indexing cupcfd_gpu_mesh::prefetchWave
-enum PfKernel { PF_FWD_F32 = 0, PF_ADJ_F32, PF_FWD_F64, PF_ADJ_F64, PF_FWD_MADJ, PF_GADJ, PF_MADJ, PF_COUNT };
+enum PfKernel {
+    PF_FWD_F32 = 0, PF_ADJ_F32, PF_FWD_F64, PF_ADJ_F64, PF_FWD_MADJ, PF_GADJ, PF_MADJ, PF_MADJ_F64,
+    PF_GRAD_F64, PF_GRAD_F32, PF_CORR_F64, PF_CORR_F32, PF_GRAD_ADJ_F64, PF_GRAD_ADJ_F32, PF_COUNT
+};
 
 // scratch slots of a mesh (each grows on demand and is reused across calls)
 enum Slot {
@@ -116,6 +119,14 @@ class KernelTimer {
 };
 #define KTIMER(name, stream) KernelTimer ktimer_(name, stream)
 
+// the kernel templates of more than the list form, by that alone
+template <int WF> constexpr auto k_grad_f64_pf = k_grad_pf<double, false, WF>;
+template <int WF> constexpr auto k_grad_f32_pf = k_grad_pf<float, false, WF>;
+template <int WF> constexpr auto k_corr_f64_pf = k_grad_pf<double, true, WF>;
+template <int WF> constexpr auto k_corr_f32_pf = k_grad_pf<float, true, WF>;
+template <int WF> constexpr auto k_grad_adj_f64_pf = k_grad_adj_pf<double, WF>;
+template <int WF> constexpr auto k_grad_adj_f32_pf = k_grad_adj_pf<float, WF>;
+
 inline bool aligned16(const void *p) { return ((uintptr_t) p & 15u) == 0; }
 
 // Builds the per-tile ranges the L2-prefetch kernels of both precisions read
@@ -171,21 +182,32 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
         PF_KERNEL(k_adj_f64_pf),
         PF_KERNEL(k_fwd_madj_f32_pf),
         PF_KERNEL(k_gadj_f32_pf),
-        PF_KERNEL(k_madj_f32_pf)};
+        PF_KERNEL(k_madj_f32_pf),
+        PF_KERNEL(k_madj_f64_pf),
+        PF_KERNEL(k_grad_f64_pf),
+        PF_KERNEL(k_grad_f32_pf),
+        PF_KERNEL(k_corr_f64_pf),
+        PF_KERNEL(k_corr_f32_pf),
+        PF_KERNEL(k_grad_adj_f64_pf),
+        PF_KERNEL(k_grad_adj_f32_pf)};
 #undef PF_KERNEL
     static_assert(sizeof(pfKern) / sizeof(pfKern[0]) == PF_COUNT, "one kernel per PfKernel");
     static_assert(PF_COUNT <= (int) (sizeof(m->prefetchWave) / sizeof(m->prefetchWave[0])), "room for every wave");
 #define PF_BLOCK(B) (wf == -6 ? B<-6> : wf == 6 ? B<6> : B<0>)
     const int pfBlock[PF_COUNT] = {PF_BLOCK(PF_BLOCK_FWD),      PF_BLOCK(PF_BLOCK_ADJ),  PF_BLOCK(PF_BLOCK_FWD_F64), PF_BLOCK(PF_BLOCK_ADJ_F64),
-                                   PF_BLOCK(PF_BLOCK_FWD_MADJ), PF_BLOCK(PF_BLOCK_GADJ), PF_BLOCK(PF_BLOCK_MADJ)};
+                                   PF_BLOCK(PF_BLOCK_FWD_MADJ), PF_BLOCK(PF_BLOCK_GADJ), PF_BLOCK(PF_BLOCK_MADJ),
+                                   PF_BLOCK(PF_BLOCK_MADJ_F64), PF_BLOCK(PF_BLOCK_GRAD), PF_BLOCK(PF_BLOCK_GRAD),
+                                   PF_BLOCK(PF_BLOCK_GRAD), PF_BLOCK(PF_BLOCK_GRAD), PF_BLOCK(PF_BLOCK_GRAD_ADJ),
+                                   PF_BLOCK(PF_BLOCK_GRAD_ADJ)};
 #undef PF_BLOCK
     // prefetch distance in waves, in quarters, measured at 256^3 (same box):
     // 1.25 waves for the forward+mass adjoint (0.538 ms against 0.546 at 1
     // wave, 0.541 at 1.5, 0.581 at 0.75), the separate FP32 forward and
     // adjoint (0.491 / 0.528 against 0.492 / 0.531), the FP64 forward (0.706
     // against 0.720) and the mass-only adjoint; 1 wave for the gradient
-    // adjoint (equal) and the FP64 adjoint (0.84 against 0.81 ms)
-    int pfQuarters[PF_COUNT] = {5, 5, 5, 4, 5, 4, 5};
+    // adjoint (equal) and the FP64 adjoint (0.84 against 0.81 ms); the
+    // gradient kernels as the forward
+    int pfQuarters[PF_COUNT] = {5, 5, 5, 4, 5, 4, 5, 5, 5, 5, 5, 5, 5, 5};
     // CUPCFD_PREFETCH_QUARTERS=q sets every kernel's distance to q/4 waves
     if (const char *e = std::getenv("CUPCFD_PREFETCH_QUARTERS"))
         if (*e)
@@ -255,6 +277,23 @@ int launch_grad_once(cupcfd_gpu_mesh *m, int precision, bool corr, bool sgn, con
                      const void *prev, void *grad, void *gcopy, cudaStream_t st) {
     int64_t ldc = m->nC;
     unsigned grid = grid_for(m->nC, BLK);
+    // the reference's sign on tiled meshes and 16-byte aligned arrays: the
+    // L2-prefetch kernels (the same bits)
+    if (m->tiles && !sgn && precision != CUPCFD_PREC_F32REF && aligned16(phi) && aligned16(prev)) {
+#define GRAD_PF(T, G, C, PHI, K, BLOCK, W)                                                                            \
+    CG_LAUNCH_PF(m, K, BLOCK, st, m->nC, sell(m), m->G, m->C, m->PHI, (const T *) phi, (const T *) phiB, m->vol,       \
+                 (const T *) prev, (T *) grad, (T *) gcopy, ldc, prefetch_args(m, W))
+        if (precision == CUPCFD_PREC_F64) {
+            if (corr) GRAD_PF(double, fg64, fc64, cc64, k_corr_f64_pf, PF_BLOCK_GRAD, PF_CORR_F64);
+            else GRAD_PF(double, fg64, fc64, cc64, k_grad_f64_pf, PF_BLOCK_GRAD, PF_GRAD_F64);
+        } else {
+            if (corr) GRAD_PF(float, fg32, fc32, cc32, k_corr_f32_pf, PF_BLOCK_GRAD, PF_CORR_F32);
+            else GRAD_PF(float, fg32, fc32, cc32, k_grad_f32_pf, PF_BLOCK_GRAD, PF_GRAD_F32);
+        }
+#undef GRAD_PF
+        CG_LAUNCHED();
+        return CUPCFD_E_SUCCESS;
+    }
     if (precision == CUPCFD_PREC_F64) {
         const double *pp = (const double *) phi, *pb = (const double *) phiB, *go = (const double *) prev;
         double *g = (double *) grad, *gc = (double *) gcopy;
@@ -369,18 +408,18 @@ extern "C" int cupcfd_gpu_dev_gradient(cupcfd_gpu_mesh *m, int32_t precision, in
         if (grad_o) CG_CHECK_CUDA(cudaMemsetAsync(grad_o, 0, bytes, st));
         return CUPCFD_E_SUCCESS;
     }
-    // first iteration: the previous iterate is zero, so the correction is exactly +0 and skipped
-    CG_TRY(launch_grad_once(m, precision, false, sgn, phi, phiB, nullptr, grad, nGradient == 1 ? grad_o : nullptr, st));
-    if (nGradient > 1) {
-        // later iterations read the previous iterate from a separate copy so
-        // no launch reads the buffer it writes
-        char *prev;
-        CG_TRY(scratch(m, S_GO, bytes, &prev));
-        for (int it = 1; it < nGradient; it++) {
-            CG_CHECK_CUDA(cudaMemcpyAsync(prev, grad, bytes, cudaMemcpyDeviceToDevice, st));
-            CG_TRY(launch_grad_once(m, precision, true, sgn, phi, phiB, prev, grad, nullptr, st));
-        }
-        if (grad_o) CG_CHECK_CUDA(cudaMemcpyAsync(grad_o, grad, bytes, cudaMemcpyDeviceToDevice, st));
+    // The first iteration's previous iterate is zero, so its correction is
+    // exactly +0 and skipped. Later ones read the one before from the other of
+    // two buffers (no launch reads what it writes), so that the last lands in
+    // grad; it also fills grad_o.
+    char *other = nullptr;
+    if (nGradient > 1) CG_TRY(scratch(m, S_GO, bytes, &other));
+    const void *prev = nullptr;
+    for (int it = 0; it < nGradient; it++) {
+        const bool last = it == nGradient - 1;
+        void *to = (nGradient - 1 - it) % 2 == 0 ? grad : other;
+        CG_TRY(launch_grad_once(m, precision, it > 0, sgn, phi, phiB, prev, to, last ? grad_o : nullptr, st));
+        prev = to;
     }
     return CUPCFD_E_SUCCESS;
 }
@@ -409,13 +448,20 @@ extern "C" int cupcfd_gpu_dev_gradient_adjoint(cupcfd_gpu_mesh *m, int32_t preci
                  "unknown sign_mode");
     cudaStream_t st = as_stream(stream);
     unsigned grid = grid_for(m->nC, BLK);
-    bool sgn = sign_mode == CUPCFD_SIGN_SIGNED;
-    if (precision == CUPCFD_PREC_F64) {
-        if (sgn) k_grad_adj_general<true, double><<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, nullptr, m->vol, (const double *) gbar, (double *) phiBar, (double *) phiBBar, m->nC);
-        else k_grad_adj_general<false, double><<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, nullptr, m->vol, (const double *) gbar, (double *) phiBar, (double *) phiBBar, m->nC);
+    const bool f64 = precision == CUPCFD_PREC_F64, sgn = sign_mode == CUPCFD_SIGN_SIGNED;
+    if (m->tiles && !sgn && aligned16(gbar)) {
+        if (f64)
+            CG_LAUNCH_PF(m, k_grad_adj_f64_pf, PF_BLOCK_GRAD_ADJ, st, m->nC, sell(m), m->fg64, m->ivol, (const double *) gbar,
+                         (double *) phiBar, (double *) phiBBar, m->nC, prefetch_args(m, PF_GRAD_ADJ_F64));
+        else
+            CG_LAUNCH_PF(m, k_grad_adj_f32_pf, PF_BLOCK_GRAD_ADJ, st, m->nC, sell(m), m->fg32, m->ivol, (const float *) gbar,
+                         (float *) phiBar, (float *) phiBBar, m->nC, prefetch_args(m, PF_GRAD_ADJ_F32));
+    } else if (f64) {
+        if (sgn) k_grad_adj<true, double><<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, m->ivol, (const double *) gbar, (double *) phiBar, (double *) phiBBar, m->nC);
+        else k_grad_adj<false, double><<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, m->ivol, (const double *) gbar, (double *) phiBar, (double *) phiBBar, m->nC);
     } else {
-        if (sgn) k_grad_adj_general<true, float><<<grid, BLK, 0, st>>>(m->nC, sell(m), nullptr, m->fg32, m->vol, (const float *) gbar, (float *) phiBar, (float *) phiBBar, m->nC);
-        else k_grad_adj_general<false, float><<<grid, BLK, 0, st>>>(m->nC, sell(m), nullptr, m->fg32, m->vol, (const float *) gbar, (float *) phiBar, (float *) phiBBar, m->nC);
+        if (sgn) k_grad_adj<true, float><<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg32, m->ivol, (const float *) gbar, (float *) phiBar, (float *) phiBBar, m->nC);
+        else k_grad_adj<false, float><<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg32, m->ivol, (const float *) gbar, (float *) phiBar, (float *) phiBBar, m->nC);
     }
     CG_LAUNCHED();
     return CUPCFD_E_SUCCESS;
@@ -429,7 +475,13 @@ extern "C" int cupcfd_gpu_dev_mass_plain_adjoint(cupcfd_gpu_mesh *m, int32_t pre
     CG_TRY(check_align(precision, {mbar}, {state, stateBar}));
     cudaStream_t st = as_stream(stream);
     unsigned grid = grid_for(m->nC, BLK);
-    if (precision == CUPCFD_PREC_F64)
+    if (m->tiles && aligned16(state) && aligned16(mbar) && precision == CUPCFD_PREC_F64)
+        CG_LAUNCH_PF(m, k_madj_f64_pf, PF_BLOCK_MADJ_F64, st, m->nC, sell(m), m->fg64, (const double *) state,
+                     (const double *) mbar, (double *) stateBar, m->nC, prefetch_args(m, PF_MADJ_F64));
+    else if (m->tiles && aligned16(mbar) && precision == CUPCFD_PREC_F32C)  // the state is 16-byte aligned (check_align)
+        CG_LAUNCH_PF(m, k_madj_f32_pf, PF_BLOCK_MADJ, st, m->nC, sell(m), m->fg32, (const float4 *) state,
+                     (const float *) mbar, (float4 *) stateBar, m->nC, prefetch_args(m, PF_MADJ));
+    else if (precision == CUPCFD_PREC_F64)
         k_adj_f64<<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, nullptr, 0.0, (const double *) state,
                                         (const double *) mbar, nullptr, nullptr, (double *) stateBar, m->nC);
     else

@@ -148,7 +148,7 @@ struct cupcfd_gpu_mesh {
     double4 *fxp64 = nullptr;  // {xpac, 0}; null when xpacZero
     double4 *fxn64 = nullptr;  // {xnac, 0}; null when xpacZero
     double4 *cc64 = nullptr;   // {xc, yc, zc, 0}
-    double *vol = nullptr;     // FP64 in both precisions
+    double *vol = nullptr, *ivol = nullptr;  // V and 1 / V, FP64 in both precisions
     // FP32 geometry
     float4 *fg32 = nullptr;
     float4 *fc32 = nullptr;
@@ -185,7 +185,7 @@ struct cupcfd_gpu_mesh {
     int nTiles = 0;
     bool tiles = false;
     int prefetchDist = 0;         // tiles ahead for the L2 prefetch
-    int prefetchWave[8] = {};  // per prefetch kernel (PfKernel in api.cu): one wave of its blocks, in tiles
+    int prefetchWave[16] = {};  // per prefetch kernel (PfKernel in api.cu): one wave of its blocks, in tiles
 
     std::vector<cupcfd_gpu::DevBuf> owned;  // everything above, freed by destroy
     std::vector<cupcfd_gpu::DevBuf> scratch; // reusable buffers for host-buffer calls

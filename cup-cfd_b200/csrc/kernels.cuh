@@ -181,6 +181,15 @@ __device__ __forceinline__ double4 ldg4(const double4 *p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 __device__ __forceinline__ float4 ldg4(const float4 *p) { return __ldg(p); }
+// a face record of T
+template <class T>
+struct Vec4 {
+    using type = float4;
+};
+template <>
+struct Vec4<double> {
+    using type = double4;
+};
 
 
 // Gathers into shared memory without a register held per value (cp.async):
@@ -224,7 +233,7 @@ __device__ __forceinline__ void stage_wait(int left) {
 // chunk loop's trip count at compile time and drops the padding tests
 // (kernels_pf.cuh).
 #ifndef CUPCFD_GRAD_CHUNK
-#define CUPCFD_GRAD_CHUNK 6
+#define CUPCFD_GRAD_CHUNK 6  // the plain gradient kernels
 #endif
 #ifndef CUPCFD_FWD_CHUNK
 #define CUPCFD_FWD_CHUNK 3
@@ -263,16 +272,14 @@ constexpr int CHUNK = CUPCFD_GRAD_CHUNK;
 // correction of the previous iterate (needed from the second iteration on;
 // with a zero previous iterate the term is exactly +0 and is skipped).
 // ---------------------------------------------------------------------------
-template <bool CORR, bool SIGNED>
-__global__ void __launch_bounds__(256, CUPCFD_MINB_F64) k_grad_f64(int nC, SellView sv, const double4 *__restrict__ fg,
-                                                  const double4 *__restrict__ fc, const double4 *__restrict__ cc,
-                                                  const double *__restrict__ phi, const double *__restrict__ phiB,
-                                                  const double *__restrict__ vol, const double *__restrict__ go,
-                                                  double *__restrict__ g, double *__restrict__ gcopy, int64_t ldc) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nC) return;
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
+template <bool CORR, bool SIGNED, int CH, int WF>
+__device__ __forceinline__ void grad_cell_f64(int c, const SellView &sv, const double4 *__restrict__ fg,
+                                              const double4 *__restrict__ fc, const double4 *__restrict__ cc,
+                                              const double *__restrict__ phi, const double *__restrict__ phiB,
+                                              const double *__restrict__ vol, const double *__restrict__ go,
+                                              double *__restrict__ g, double *__restrict__ gcopy, int64_t ldc) {
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
     double phic = phi[c];
     double4 xc = make_double4(0, 0, 0, 0);
     double gc0 = 0, gc1 = 0, gc2 = 0;
@@ -281,49 +288,49 @@ __global__ void __launch_bounds__(256, CUPCFD_MINB_F64) k_grad_f64(int nC, SellV
         gc0 = go[c]; gc1 = go[ldc + c]; gc2 = go[2 * ldc + c];
     }
     double ax = 0.0, ay = 0.0, az = 0.0;
-    for (int k0 = 0; k0 < w; k0 += CHUNK) {
-        int2 en[CHUNK];
-        load_entries(e, k0, w, en);
-        double4 G[CHUNK];
-        double pv[CHUNK];
+    for (int k0 = 0; k0 < w; k0 += CH) {
+        int2 en[CH];
+        e.load(k0, en);
+        double4 G[CH], xo[CH], xf[CH];
+        double pv[CH], gn[CH][3];
 #pragma unroll
-        for (int j = 0; j < CHUNK; j++) {
-            if (en[j].x < 0) continue;
+        for (int j = 0; j < CH; j++) {
+            if (!WF && en[j].x < 0) continue;
             G[j] = ldg4(fg + (en[j].x >> 1));
             int o = en[j].y;
             pv[j] = o >= 0 ? __ldg(phi + o) : __ldg(phiB + (-1 - o));
+            if (CORR && o >= 0) {
+                xo[j] = ldg4(cc + o);
+                xf[j] = ldg4(fc + (en[j].x >> 1));
+                gn[j][0] = __ldg(go + o); gn[j][1] = __ldg(go + ldc + o); gn[j][2] = __ldg(go + 2 * ldc + o);
+            }
         }
 #pragma unroll
-        for (int j = 0; j < CHUNK; j++) {
+        for (int j = 0; j < CH; j++) {
             int code = en[j].x;
-            if (code < 0) continue;
+            if (!WF && code < 0) continue;
             bool isN = code & 1;
-            int o = en[j].y;
             double phif;
-            if (o < 0) {
+            if (en[j].y < 0) {
                 phif = pv[j];
             } else {
-                double facn = G[j].w;
-                double facp = ds(1.0, facn);
-                double phN = isN ? phic : pv[j], phP = isN ? pv[j] : phic;
-                phif = da(dm(phN, facn), dm(phP, facp));
+                // this cell's and the other's weights: facn weights cell2 (N),
+                // facp cell1 (P); x_N facn + x_P facp is x_o wo + x_c wc for
+                // either role (IEEE addition commutes exactly)
+                const double facn = G[j].w, facp = ds(1.0, facn);
+                const double wo = isN ? facp : facn, wc = isN ? facn : facp;
+                phif = da(dm(pv[j], wo), dm(phic, wc));
                 if (CORR) {
-                    double4 xo = ldg4(cc + o);
-                    double4 xf = ldg4(fc + (code >> 1));
-                    double go0 = __ldg(go + o), go1 = __ldg(go + ldc + o), go2 = __ldg(go + 2 * ldc + o);
-                    double4 xN = isN ? xc : xo, xP = isN ? xo : xc;
-                    double gN0 = isN ? gc0 : go0, gN1 = isN ? gc1 : go1, gN2 = isN ? gc2 : go2;
-                    double gP0 = isN ? go0 : gc0, gP1 = isN ? go1 : gc1, gP2 = isN ? go2 : gc2;
-                    double xac0 = da(dm(xN.x, facn), dm(xP.x, facp));
-                    double xac1 = da(dm(xN.y, facn), dm(xP.y, facp));
-                    double xac2 = da(dm(xN.z, facn), dm(xP.z, facp));
-                    double ga0 = da(dm(gN0, facn), dm(gP0, facp));
-                    double ga1 = da(dm(gN1, facn), dm(gP1, facp));
-                    double ga2 = da(dm(gN2, facn), dm(gP2, facp));
+                    const double xac0 = da(dm(xo[j].x, wo), dm(xc.x, wc));
+                    const double xac1 = da(dm(xo[j].y, wo), dm(xc.y, wc));
+                    const double xac2 = da(dm(xo[j].z, wo), dm(xc.z, wc));
+                    const double ga0 = da(dm(gn[j][0], wo), dm(gc0, wc));
+                    const double ga1 = da(dm(gn[j][1], wo), dm(gc1, wc));
+                    const double ga2 = da(dm(gn[j][2], wo), dm(gc2, wc));
                     double d = 0.0;
-                    d = da(d, dm(ga0, ds(xf.x, xac0)));
-                    d = da(d, dm(ga1, ds(xf.y, xac1)));
-                    d = da(d, dm(ga2, ds(xf.z, xac2)));
+                    d = da(d, dm(ga0, ds(xf[j].x, xac0)));
+                    d = da(d, dm(ga1, ds(xf[j].y, xac1)));
+                    d = da(d, dm(ga2, ds(xf[j].z, xac2)));
                     phif = da(phif, d);
                 }
             }
@@ -340,19 +347,28 @@ __global__ void __launch_bounds__(256, CUPCFD_MINB_F64) k_grad_f64(int nC, SellV
     if (gcopy) { gcopy[c] = ax; gcopy[ldc + c] = ay; gcopy[2 * ldc + c] = az; }
 }
 
+// Without the L2 prefetch: any numbering, alignment and sign mode.
+template <bool CORR, bool SIGNED>
+__global__ void __launch_bounds__(256, CUPCFD_MINB_F64) k_grad_f64(int nC, SellView sv, const double4 *__restrict__ fg,
+                                                  const double4 *__restrict__ fc, const double4 *__restrict__ cc,
+                                                  const double *__restrict__ phi, const double *__restrict__ phiB,
+                                                  const double *__restrict__ vol, const double *__restrict__ go,
+                                                  double *__restrict__ g, double *__restrict__ gcopy, int64_t ldc) {
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < nC) grad_cell_f64<CORR, SIGNED, CORR ? 2 : CHUNK, 0>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
+}
+
 // ---------------------------------------------------------------------------
 // Gradient, FP32 storage and arithmetic, compensated accumulation (Acc2), FP64 1/V.
 // ---------------------------------------------------------------------------
-template <bool CORR, bool SIGNED>
-__global__ void __launch_bounds__(256, CUPCFD_MINB_F32) k_grad_f32(int nC, SellView sv, const float4 *__restrict__ fg,
-                                                  const float4 *__restrict__ fc, const float4 *__restrict__ cc,
-                                                  const float *__restrict__ phi, const float *__restrict__ phiB,
-                                                  const double *__restrict__ vol, const float *__restrict__ go,
-                                                  float *__restrict__ g, float *__restrict__ gcopy, int64_t ldc) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nC) return;
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
+template <bool CORR, bool SIGNED, int CH, int WF>
+__device__ __forceinline__ void grad_cell_f32(int c, const SellView &sv, const float4 *__restrict__ fg,
+                                              const float4 *__restrict__ fc, const float4 *__restrict__ cc,
+                                              const float *__restrict__ phi, const float *__restrict__ phiB,
+                                              const double *__restrict__ vol, const float *__restrict__ go,
+                                              float *__restrict__ g, float *__restrict__ gcopy, int64_t ldc) {
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
     float phic = phi[c];
     float4 xc = make_float4(0, 0, 0, 0);
     float gc0 = 0, gc1 = 0, gc2 = 0;
@@ -361,41 +377,46 @@ __global__ void __launch_bounds__(256, CUPCFD_MINB_F32) k_grad_f32(int nC, SellV
         gc0 = go[c]; gc1 = go[ldc + c]; gc2 = go[2 * ldc + c];
     }
     Acc2 ax, ay, az;
-    for (int k0 = 0; k0 < w; k0 += CHUNK) {
-        int2 en[CHUNK];
-        load_entries(e, k0, w, en);
-        float4 G[CHUNK];
-        float pv[CHUNK];
+    for (int k0 = 0; k0 < w; k0 += CH) {
+        int2 en[CH];
+        e.load(k0, en);
+        float4 G[CH], xo[CH], xf[CH];
+        float pv[CH], gn[CH][3];
 #pragma unroll
-        for (int j = 0; j < CHUNK; j++) {
-            if (en[j].x < 0) continue;
+        for (int j = 0; j < CH; j++) {
+            if (!WF && en[j].x < 0) continue;
             G[j] = __ldg(fg + (en[j].x >> 1));
             int o = en[j].y;
             pv[j] = o >= 0 ? __ldg(phi + o) : __ldg(phiB + (-1 - o));
+            if (CORR && o >= 0) {
+                xo[j] = __ldg(cc + o);
+                xf[j] = __ldg(fc + (en[j].x >> 1));
+                gn[j][0] = __ldg(go + o); gn[j][1] = __ldg(go + ldc + o); gn[j][2] = __ldg(go + 2 * ldc + o);
+            }
         }
 #pragma unroll
-        for (int j = 0; j < CHUNK; j++) {
+        for (int j = 0; j < CH; j++) {
             int code = en[j].x;
-            if (code < 0) continue;
+            if (!WF && code < 0) continue;
             bool isN = code & 1;
-            int o = en[j].y;
             float phif;
-            if (o < 0) {
+            if (en[j].y < 0) {
                 phif = pv[j];
             } else {
                 float facn = G[j].w, facp = 1.f - facn;
                 phif = interp(face_weights(facn, isN), phic, pv[j]);
                 if (CORR) {
-                    float4 xo = __ldg(cc + o), xf = __ldg(fc + (code >> 1));
-                    float go0 = __ldg(go + o), go1 = __ldg(go + ldc + o), go2 = __ldg(go + 2 * ldc + o);
-                    float4 xN = isN ? xc : xo, xP = isN ? xo : xc;
-                    float gN0 = isN ? gc0 : go0, gN1 = isN ? gc1 : go1, gN2 = isN ? gc2 : go2;
-                    float gP0 = isN ? go0 : gc0, gP1 = isN ? go1 : gc1, gP2 = isN ? go2 : gc2;
-                    float d0 = xf.x - fmaf(facn, xN.x, facp * xP.x);
-                    float d1 = xf.y - fmaf(facn, xN.y, facp * xP.y);
-                    float d2 = xf.z - fmaf(facn, xN.z, facp * xP.z);
-                    phif += fmaf(facn, gN0, facp * gP0) * d0 + fmaf(facn, gN1, facp * gP1) * d1 +
-                            fmaf(facn, gN2, facp * gP2) * d2;
+                    float4 xN = isN ? xc : xo[j], xP = isN ? xo[j] : xc;
+                    float gN0 = isN ? gc0 : gn[j][0], gN1 = isN ? gc1 : gn[j][1], gN2 = isN ? gc2 : gn[j][2];
+                    float gP0 = isN ? gn[j][0] : gc0, gP1 = isN ? gn[j][1] : gc1, gP2 = isN ? gn[j][2] : gc2;
+                    // explicit roundings: the plain and the L2-prefetch kernels then give the same bits
+                    float d0 = __fsub_rn(xf[j].x, __fmaf_rn(facn, xN.x, __fmul_rn(facp, xP.x)));
+                    float d1 = __fsub_rn(xf[j].y, __fmaf_rn(facn, xN.y, __fmul_rn(facp, xP.y)));
+                    float d2 = __fsub_rn(xf[j].z, __fmaf_rn(facn, xN.z, __fmul_rn(facp, xP.z)));
+                    float a0 = __fmaf_rn(facn, gN0, __fmul_rn(facp, gP0));
+                    float a1 = __fmaf_rn(facn, gN1, __fmul_rn(facp, gP1));
+                    float a2 = __fmaf_rn(facn, gN2, __fmul_rn(facp, gP2));
+                    phif = __fadd_rn(phif, __fmaf_rn(a2, d2, __fmaf_rn(a1, d1, __fmul_rn(a0, d0))));
                 }
             }
             if (SIGNED && isN) {
@@ -409,6 +430,17 @@ __global__ void __launch_bounds__(256, CUPCFD_MINB_F32) k_grad_f32(int nC, SellV
     float rx = (float) (ax.value() * fact), ry = (float) (ay.value() * fact), rz = (float) (az.value() * fact);
     g[c] = rx; g[ldc + c] = ry; g[2 * ldc + c] = rz;
     if (gcopy) { gcopy[c] = rx; gcopy[ldc + c] = ry; gcopy[2 * ldc + c] = rz; }
+}
+
+// Without the L2 prefetch: any numbering, alignment and sign mode.
+template <bool CORR, bool SIGNED>
+__global__ void __launch_bounds__(256, CUPCFD_MINB_F32) k_grad_f32(int nC, SellView sv, const float4 *__restrict__ fg,
+                                                  const float4 *__restrict__ fc, const float4 *__restrict__ cc,
+                                                  const float *__restrict__ phi, const float *__restrict__ phiB,
+                                                  const double *__restrict__ vol, const float *__restrict__ go,
+                                                  float *__restrict__ g, float *__restrict__ gcopy, int64_t ldc) {
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < nC) grad_cell_f32<CORR, SIGNED, CORR ? 2 : CHUNK, 0>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
 }
 
 // ---------------------------------------------------------------------------

@@ -667,39 +667,61 @@ __global__ void __launch_bounds__(256, CUPCFD_MINB_F32) k_adj_f32(int nC, SellVi
     if (c < nC) adj_cell_f32<false>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
 }
 
-// General gradient adjoint (input gbar = dL/dg, any loss): h_c = gbar_c / V_c.
-template <bool SIGNED, class T>
-__global__ void __launch_bounds__(256) k_grad_adj_general(int nC, SellView sv, const double4 *__restrict__ fg64,
-                                                          const float4 *__restrict__ fg32, const double *__restrict__ vol,
-                                                          const T *__restrict__ gbar, T *__restrict__ phibar,
-                                                          T *__restrict__ phibBar, int64_t ldc) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nC) return;
-    int w;
-    const int2 *e = cell_entries(sv, c, w);
-    double iv = 1.0 / vol[c];
-    double hx = (double) gbar[c] * iv, hy = (double) gbar[ldc + c] * iv, hz = (double) gbar[2 * ldc + c] * iv;
+// General gradient adjoint (input gbar = dL/dg, any loss): h_c = gbar_c / V_c
+// (ivol = 1 / V, kept with the mesh: six divisions per cell fewer). FP64
+// arithmetic on T's geometry and fields.
+template <bool SIGNED, class T, int CH, int WF>
+__device__ __forceinline__ void grad_adj_cell(int c, const SellView &sv, const typename Vec4<T>::type *__restrict__ fg,
+                                              const double *__restrict__ ivol, const T *__restrict__ gbar,
+                                              T *__restrict__ phibar, T *__restrict__ phibBar, int64_t ldc) {
+    const CellList<WF> e(sv, c);
+    const int w = e.w;
+    const double iv = ivol[c];
+    const double hx = __dmul_rn((double) gbar[c], iv), hy = __dmul_rn((double) gbar[ldc + c], iv),
+                 hz = __dmul_rn((double) gbar[2 * ldc + c], iv);
     double pb = 0.0;
-    for (int k = 0; k < w; k++) {
-        int2 en = __ldg(e + 32 * k);
-        if (en.x < 0) break;
-        int f = en.x >> 1, o = en.y;
-        bool isN = en.x & 1;
-        double Sx, Sy, Sz, lam;
-        if (fg64) { double4 G = ldg4(fg64 + f); Sx = G.x; Sy = G.y; Sz = G.z; lam = G.w; }
-        else { float4 G = __ldg(fg32 + f); Sx = G.x; Sy = G.y; Sz = G.z; lam = G.w; }
-        double own = hx * Sx + hy * Sy + hz * Sz;
-        if (o < 0) {
-            phibBar[-1 - o] = (T) own;
-            continue;
+    for (int k0 = 0; k0 < w; k0 += CH) {
+        int2 en[CH];
+        e.load(k0, en);
+        typename Vec4<T>::type G[CH];
+        T go[CH][3];
+        double io[CH];
+#pragma unroll
+        for (int j = 0; j < CH; j++) {
+            if (!WF && en[j].x < 0) continue;
+            const int o = en[j].y;
+            G[j] = ldg4(fg + (en[j].x >> 1));
+            if (o < 0) continue;
+            go[j][0] = __ldg(gbar + o); go[j][1] = __ldg(gbar + ldc + o); go[j][2] = __ldg(gbar + 2 * ldc + o);
+            io[j] = __ldg(ivol + o);
         }
-        double ivo = 1.0 / __ldg(vol + o);
-        double oth = ((double) gbar[o] * Sx + (double) gbar[ldc + o] * Sy + (double) gbar[2 * ldc + o] * Sz) * ivo;
-        // d g_P / d phi_f = +S/V_P; d g_N / d phi_f = +S/V_N (reference) or -S/V_N (signed)
-        double sOwn = (SIGNED && isN) ? -1.0 : 1.0, sOth = (SIGNED && !isN) ? -1.0 : 1.0;
-        pb += (isN ? lam : 1.0 - lam) * (sOwn * own + sOth * oth);
+#pragma unroll
+        for (int j = 0; j < CH; j++) {
+            if (!WF && en[j].x < 0) continue;
+            const int o = en[j].y;
+            const bool isN = en[j].x & 1;
+            const double Sx = G[j].x, Sy = G[j].y, Sz = G[j].z, lam = G[j].w;
+            const double own = __fma_rn(hz, Sz, __fma_rn(hy, Sy, __dmul_rn(hx, Sx)));
+            if (o < 0) {
+                phibBar[-1 - o] = (T) own;
+                continue;
+            }
+            const double oth = __dmul_rn(__fma_rn((double) go[j][2], Sz, __fma_rn((double) go[j][1], Sy, __dmul_rn((double) go[j][0], Sx))), io[j]);
+            // d g_P / d phi_f = +S/V_P; d g_N / d phi_f = +S/V_N (reference) or -S/V_N (signed)
+            const double sum = SIGNED ? (isN ? __dsub_rn(oth, own) : __dsub_rn(own, oth)) : __dadd_rn(own, oth);
+            pb = __fma_rn(isN ? lam : __dsub_rn(1.0, lam), sum, pb);
+        }
     }
     phibar[c] = (T) pb;
+}
+
+// Without the L2 prefetch: any numbering, alignment and sign mode.
+template <bool SIGNED, class T>
+__global__ void __launch_bounds__(256) k_grad_adj(int nC, SellView sv, const typename Vec4<T>::type *__restrict__ fg,
+                                                  const double *__restrict__ ivol, const T *__restrict__ gbar,
+                                                  T *__restrict__ phibar, T *__restrict__ phibBar, int64_t ldc) {
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < nC) grad_adj_cell<SIGNED, T, 2, 0>(c, sv, fg, ivol, gbar, phibar, phibBar, ldc);
 }
 
 // ---------------------------------------------------------------------------

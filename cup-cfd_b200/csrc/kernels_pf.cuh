@@ -24,6 +24,24 @@ template <int WF> constexpr int PF_BLOCK_ADJ_F64 = 128;
 template <int WF> constexpr int PF_BLOCK_FWD_MADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_GADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_MADJ = 256;
+template <int WF> constexpr int PF_BLOCK_MADJ_F64 = 128;
+template <int WF> constexpr int PF_BLOCK_GRAD = 128;
+template <int WF> constexpr int PF_BLOCK_GRAD_ADJ = 128;
+
+// Entries per chunk of the gradient kernels, and the tiles' worth of blocks
+// per SM the registers allow. At 128^3 (112^3 permuted for the correction),
+// all in 128-thread blocks: one FP64 gradient 56 us at 2 / 4 (3 / 4 60, 1 / 6
+// 59, 6 / 3 in 256-thread blocks 68), against 106 for the plain kernel. An
+// iteration with the correction carries fourteen values per face: three
+// iterations on the permuted mesh 352 us at 2 / 2 (110 registers; 1 / 3 374,
+// 1 / 4 spilling 451) against 449 for the plain kernels with a copy after each
+// iteration; on rows in run form 314 at 1 / 3, 333 at 2 / 2, against 527. The
+// general adjoint 3 / 3: with the mass adjoint 154 us, 2 / 4 156, 1 / 4 160,
+// against 241 (its plain kernel took the incidences one by one, with a
+// division each).
+template <bool CORR, int WF> constexpr int PF_CHUNK_GRAD = CORR && WF == -6 ? 1 : 2;
+template <bool CORR, int WF> constexpr int PF_MINB_GRAD = CORR ? (WF == -6 ? 3 : 2) : 4;
+constexpr int PF_CHUNK_GRAD_ADJ = 3, PF_MINB_GRAD_ADJ = 3;
 
 // ---------------------------------------------------------------------------
 // L2 prefetch variant: the unstaged one-cell-per-thread kernels (the same
@@ -230,6 +248,72 @@ __global__ void __launch_bounds__(PF_BLOCK_MADJ<WF>, CUPCFD_MINB_F32 *TILE_CELLS
     if (c < nC)
         adj_cell_f32<false, CUPCFD_ADJ_CHUNK, 0, WF>(c, sv, fg, nullptr, 0.f, st, gface, nullptr, nullptr, stbar, ldc);
     if (tb.lead) prefetch_tile<1>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
+}
+
+// The mass-flux part of the adjoint only, FP64 (adj_cell_f64 with hscale 0).
+template <int WF>
+__global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, CUPCFD_MINB_ADJ_F64 *TILE_CELLS / PF_BLOCK_MADJ_F64<WF>)
+    k_madj_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ st,
+                  const double *__restrict__ gface, double *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
+    constexpr int T = TILE_CELLS;
+    const TileBlock<PF_BLOCK_MADJ_F64<WF>> tb(pf);
+    const int c = tb.c;
+    __shared__ int4 s_rng;
+    const void *const cellSrc[4] = {st, st + ldc, st + 2 * ldc, st + 3 * ldc};
+    const int cellBytes[4] = {T * 8, T * 8, T * 8, T * 8};
+    if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
+    if (c < nC)
+        adj_cell_f64<false, CUPCFD_ADJ_CHUNK_F64, WF>(c, sv, fg, nullptr, 0.0, st, gface, nullptr, nullptr, stbar, ldc);
+    if (tb.lead) prefetch_tile<4>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
+}
+
+// The gradient by itself (grad_cell_*, reference sign), with the L2 prefetch;
+// CORR: an iteration with the non-orthogonal correction, which reads the
+// previous iterate go and the cells' and faces' centres as well.
+template <class T, bool CORR, int WF>
+__global__ void __launch_bounds__(PF_BLOCK_GRAD<WF>, PF_MINB_GRAD<CORR, WF> *TILE_CELLS / PF_BLOCK_GRAD<WF>)
+    k_grad_pf(int nC, SellView sv, const typename Vec4<T>::type *__restrict__ fg, const typename Vec4<T>::type *__restrict__ fc,
+              const typename Vec4<T>::type *__restrict__ cc, const T *__restrict__ phi, const T *__restrict__ phiB,
+              const double *__restrict__ vol, const T *__restrict__ go, T *__restrict__ g, T *__restrict__ gcopy, int64_t ldc,
+              PrefetchArgs pf) {
+    constexpr int TC = TILE_CELLS, S = (int) sizeof(T), N = CORR ? 6 : 2;
+    const TileBlock<PF_BLOCK_GRAD<WF>> tb(pf);
+    const int c = tb.c;
+    __shared__ int4 s_rng;
+    if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
+    if (c < nC) {
+        if constexpr (S == 8)
+            grad_cell_f64<CORR, false, PF_CHUNK_GRAD<CORR, WF>, WF>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
+        else
+            grad_cell_f32<CORR, false, PF_CHUNK_GRAD<CORR, WF>, WF>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
+    }
+    if (tb.lead) {
+        const int4 r = ranges_ready(&s_rng);
+        const void *const cellSrc[6] = {phi, vol, go, go + ldc, go + 2 * ldc, cc};
+        const int cellBytes[6] = {TC * S, TC * 8, TC * S, TC * S, TC * S, TC * 4 * S};
+        const void *src[N];
+        int bytes[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) { src[i] = cellSrc[i]; bytes[i] = cellBytes[i]; }
+        prefetch_tile<N>(pf, tb.tp, r, fg, 4 * S, (const T *) nullptr, src, bytes);
+        if (CORR && r.w > r.z) bulk_prefetch_l2(fc + r.z, (unsigned) (r.w - r.z) * (unsigned) (4 * S));
+    }
+}
+
+// The general gradient adjoint (grad_adj_cell, reference sign), with the L2 prefetch.
+template <class T, int WF>
+__global__ void __launch_bounds__(PF_BLOCK_GRAD_ADJ<WF>, PF_MINB_GRAD_ADJ *TILE_CELLS / PF_BLOCK_GRAD_ADJ<WF>)
+    k_grad_adj_pf(int nC, SellView sv, const typename Vec4<T>::type *__restrict__ fg, const double *__restrict__ ivol,
+                  const T *__restrict__ gbar, T *__restrict__ phibar, T *__restrict__ phibBar, int64_t ldc, PrefetchArgs pf) {
+    constexpr int TC = TILE_CELLS, S = (int) sizeof(T);
+    const TileBlock<PF_BLOCK_GRAD_ADJ<WF>> tb(pf);
+    const int c = tb.c;
+    __shared__ int4 s_rng;
+    const void *const cellSrc[4] = {gbar, gbar + ldc, gbar + 2 * ldc, ivol};
+    const int cellBytes[4] = {TC * S, TC * S, TC * S, TC * 8};
+    if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
+    if (c < nC) grad_adj_cell<false, T, PF_CHUNK_GRAD_ADJ, WF>(c, sv, fg, ivol, gbar, phibar, phibBar, ldc);
+    if (tb.lead) prefetch_tile<4>(pf, tb.tp, ranges_ready(&s_rng), fg, 4 * S, (const T *) nullptr, cellSrc, cellBytes);
 }
 
 // Largest |c - neighbour| over the incidence lists (the numbering's bandwidth).

@@ -204,7 +204,7 @@ __global__ void k_layout_faces(int nF, const int *__restrict__ faceN2O, const in
 
 __global__ void k_layout_cells(int nC, const int *__restrict__ cellN2O, const double *__restrict__ cc,
                                const double *__restrict__ vol, double4 *__restrict__ cc64, float4 *__restrict__ cc32,
-                               double *__restrict__ vout) {
+                               double *__restrict__ vout, double *__restrict__ ivout) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nC) return;
     int o = cellN2O[c];
@@ -212,6 +212,7 @@ __global__ void k_layout_cells(int nC, const int *__restrict__ cellN2O, const do
     if (cc64) cc64[c] = p;
     if (cc32) cc32[c] = make_float4((float) p.x, (float) p.y, (float) p.z, 0.f);
     vout[c] = vol[o];
+    ivout[c] = __ddiv_rn(1.0, vol[o]);
 }
 
 // one warp per slice: width = max degree over the slice's cells
@@ -708,11 +709,12 @@ int build_mesh_from_source(cupcfd_gpu_mesh *m, const Source &s, const cupcfd_mes
         CG_TRY(m->alloc(&m->cc32, (size_t) nC));
     }
     CG_TRY(m->alloc(&m->vol, (size_t) nC));
+    CG_TRY(m->alloc(&m->ivol, (size_t) nC));
     k_layout_faces<<<grid_for(nF, B), B, 0, st>>>(nF, m->faceN2O, m->cellO2N, s.c1, s.c2, s.bnd, s.lam, s.area, s.S,
                                                  s.xf, s.xpac, s.xnac, m->faceCells, m->fg64, m->fc64, m->fxp64,
                                                  m->fxn64, m->fg32, m->fc32);
     CG_LAUNCHED();
-    k_layout_cells<<<grid_for(nC, B), B, 0, st>>>(nC, m->cellN2O, s.cc, s.vol, m->cc64, m->cc32, m->vol);
+    k_layout_cells<<<grid_for(nC, B), B, 0, st>>>(nC, m->cellN2O, s.cc, s.vol, m->cc64, m->cc32, m->vol, m->ivol);
     CG_LAUNCHED();
 
     // --- SELL-32 incidence lists

@@ -359,3 +359,50 @@ def test_any_cell_count_takes_the_prefetch_kernels(cg, gpu, kind, dims, order):
         assert {"k_fwd_madj_f32_pf", "k_gadj_f32_pf"} <= set(cg.timing_read())
     finally:
         cg.timing_enable(False)
+
+
+@pytest.mark.parametrize("kind,dims,order", CASES + [("structgen", (33, 12, 7), "ORDER_OWNER"), ("poly", (9, 8, 7), "ORDER_OWNER")])
+@pytest.mark.parametrize("prec", ["PREC_F64", "PREC_F32C"])
+def test_gradient_and_general_adjoints_prefetch_equals_plain(cg, gpu, kind, dims, order, prec):
+    """dev_gradient (one to three iterations), dev_gradient_adjoint and
+    dev_mass_plain_adjoint on arrays at 16-byte boundaries (L2-prefetch
+    kernels) and off them (plain kernels): the same bits."""
+    import torch
+    if kind == "poly":
+        import oracle as O
+        mesh = cg.Mesh.from_arrays(O.merge_cells(O.jitter(*dims, 0.25, seed=5, permute=True), 0.4, 11, max_cells=6),
+                                   order=getattr(cg, order))
+    else:
+        mesh = _mesh(cg, kind, dims, order)
+    p = getattr(cg, prec)
+    f64 = p == cg.PREC_F64
+    t = torch.float64 if f64 else torch.float32
+    nC, nF, nB = mesh.nCells, mesh.nFaces, mesh.nBoundaries
+    phi, phiB, st, gface = (x.to(t) for x in _fields(torch, mesh, 29))
+    st = st.t().contiguous() if f64 else st
+    gbar = torch.randn(3, nC, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda", dtype=t)
+
+    def off(x):   # one element past a 16-byte boundary
+        buf = torch.empty(x.numel() + 4, dtype=x.dtype, device=x.device)
+        v = buf[1:1 + x.numel()].view(x.shape)
+        v.copy_(x)
+        return v
+
+    e = lambda *n: torch.full(n, float("nan"), dtype=t, device="cuda")  # noqa: E731
+    s = torch.cuda.current_stream()
+    outs = []
+    for at in (lambda x: x, off):
+        o = []
+        for n in (1, 2, 3):
+            g, go = e(3, nC), e(3, nC)
+            cg.dev_gradient(mesh, p, at(phi), phiB, g, go, nGradient=n, stream=s)
+            assert torch.equal(g, go)
+            o.append(g)
+        pb, pbb, sb = e(nC), e(nB), torch.full_like(st, float("nan"))
+        cg.dev_gradient_adjoint(mesh, p, at(gbar), pb, pbb, stream=s)
+        cg.dev_mass_plain_adjoint(mesh, p, st, at(gface), sb, stream=s)
+        mesh.check_status()
+        torch.cuda.synchronize()
+        outs.append(o + [pb, pbb, sb])
+    for a, b in zip(*outs):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
