@@ -177,10 +177,19 @@ enum UvwKind : int {
     UVW_WALLSYM = 4  // symmetry / wall: a = a + X; s = (s + X*u) - force       (:424-431, :490-497)
 };
 
+// The source of a face's carried value (the head of this file), -1 without
+// any. It leads to another load, so it is fetched while the face before is
+// computed.
+template <class T>
+__device__ __forceinline__ int uvw_carry(const UvwArgs<T> &a, int2 en) {
+    return a.carry ? __ldg(a.carry + (en.x >> 1)) : -1;
+}
+
 // The terms one incidence (entry en of cell c) contributes to its cell, and
 // the face's own outputs when c owns the face. Returns the UvwKind.
 template <class T>
-__device__ __forceinline__ int uvw_terms(const UvwArgs<T> &a, int c, const UvwOwn<T> &own, int2 en, T (&t)[10]) {
+__device__ __forceinline__ int uvw_terms(const UvwArgs<T> &a, int c, const UvwOwn<T> &own, int2 en, int carry,
+                                         T (&t)[10]) {
     using R = UvwReal<T>;
     using V4 = typename UvwReal<T>::V4;
     const int64_t L = a.ldg;
@@ -210,11 +219,10 @@ __device__ __forceinline__ int uvw_terms(const UvwArgs<T> &a, int c, const UvwOw
         const T x0 = R::sub(Cn.x, Cp.x), x1 = R::sub(Cn.y, Cp.y), x2 = R::sub(Cn.z, Cp.z);
         const T visFace = R::mul(visac, rl);
         T uF = T(0), vF = T(0), wF = T(0);
-        const int cr = a.carry ? a.carry[f] : -1;
-        if (cr >= 0) {
-            uF = a.u[cr]; vF = a.v[cr]; wF = a.w[cr];
-        } else if (cr <= -2) {
-            const double *r = a.regionUVW + 3 * (-2 - cr);
+        if (carry >= 0) {
+            uF = a.u[carry]; vF = a.v[carry]; wF = a.w[carry];
+        } else if (carry <= -2) {
+            const double *r = a.regionUVW + 3 * (-2 - carry);
             uF = (T) r[0]; vF = (T) r[1]; wF = (T) r[2];
         }
         const T mf = a.massFlux[f];
@@ -289,8 +297,7 @@ __device__ __forceinline__ int uvw_terms(const UvwArgs<T> &a, int c, const UvwOw
     T Xc, f0 = T(0), f1 = T(0), f2 = T(0);
     if (it == CUPCFD_RTYPE_SYMP) {
         // UVWKernels.ipp:383-436; visFace carried from an earlier face
-        const int g = a.carry ? a.carry[f] : -1;
-        Xc = g >= 0 ? vis_face_of(a, g) : T(0);
+        Xc = carry >= 0 ? vis_face_of(a, carry) : T(0);
         const T visac = own.vis;
         const T us0 = R::add(uc, dot0(du0, du1, du2, x0, x1, x2));
         const T us1 = R::add(vc, dot0(dv0, dv1, dv2, x0, x1, x2));
@@ -370,7 +377,7 @@ __device__ __forceinline__ void uvw_fold(int kind, const T (&t)[10], T (&s)[3], 
 // the terms staged in shared memory and one warp folding them measured
 // slower: 4.2-5.0 ms against 2.3 ms at 256^3.)
 #ifndef UVW_CELL_MINB
-#define UVW_CELL_MINB 2  // resident 256-thread blocks per SM asked of the register allocator (118 registers:
+#define UVW_CELL_MINB 2  // resident 256-thread blocks per SM asked of the register allocator (124 registers:
                          // the own-cell values held for the whole cell; 3 blocks at 80 spill them)
 #endif
 // The L2-prefetch launches run 64-thread blocks, four per 256-cell tile, at
@@ -380,25 +387,30 @@ __device__ __forceinline__ void uvw_fold(int kind, const T (&t)[10], T (&s)[3], 
 #ifndef UVW_PF_BLOCK
 #define UVW_PF_BLOCK 64
 #endif
-#ifndef UVW_CHUNK
-#define UVW_CHUNK 6      // incidence entries loaded ahead (a hexahedral cell in one chunk)
-#endif
-template <class T>
+template <class T, int WF>
 __device__ __forceinline__ void uvw_cell(const UvwArgs<T> &a, int c) {
-    int wdt;
-    const int2 *e = cell_entries(a.sv, c, wdt);
+    const CellList<WF> e(a.sv, c);
     T s[3] = {a.su[c], a.sv_[c], a.sw[c]}, ad[3] = {a.au[c], a.av[c], a.aw[c]};
     const UvwOwn<T> own = uvw_own(a, c);
-    // the chunk's entries first (independent loads), then incidence by incidence
-    for (int k0 = 0; k0 < wdt; k0 += UVW_CHUNK) {
-        int2 en[UVW_CHUNK];
-        load_entries<UVW_CHUNK>(e, k0, wdt, en);
-        for (int j = 0; j < UVW_CHUNK; j++) {
-            if (en[j].x < 0) break;
-            T t[10];
-            int kind = uvw_terms(a, c, own, en[j], t);
-            uvw_fold(kind, t, s, ad);
-        }
+    // One incidence at a time; its entry was loaded two before it and its
+    // carried value's source one before. At 160^3 with inlets, outlets, walls
+    // and symmetry planes: 427 us with the run form and 435 with the lists,
+    // 515 / 521 with the entries but not the source ahead, 616 with neither and
+    // without the prefetch of the sources and rlencos.
+    constexpr bool SIX = WF == -6;  // no padding to look for
+    auto entry = [&](int k) { return SIX ? e.at(min(k, 5)) : k < e.w ? e.at(k) : make_int2(-1, -1); };
+    int2 en = entry(0), next = entry(1);
+    int carry = SIX || en.x >= 0 ? uvw_carry(a, en) : -1;
+#pragma unroll 1
+    for (int k = 2; SIX ? k < 8 : en.x >= 0; k++) {  // a cell's padding follows its entries
+        const int carryNext = SIX || next.x >= 0 ? uvw_carry(a, next) : -1;
+        const int2 after = entry(k);
+        T t[10];
+        const int kind = uvw_terms(a, c, own, en, carry, t);
+        uvw_fold(kind, t, s, ad);
+        en = next;
+        next = after;
+        carry = carryNext;
     }
     a.su[c] = s[0]; a.sv_[c] = s[1]; a.sw[c] = s[2];
     a.au[c] = ad[0]; a.av[c] = ad[1]; a.aw[c] = ad[2];
@@ -410,7 +422,7 @@ __device__ __forceinline__ void uvw_cell(const UvwArgs<T> &a, int c) {
 // Needs the owner-sorted face order and 16-byte aligned arrays; launched as
 // UVW_PF_BLOCK-thread blocks, TILE_CELLS / UVW_PF_BLOCK per tile (the last
 // block of a tile prefetches for the tile).
-template <class T>
+template <class T, int WF>
 __device__ __forceinline__ void uvw_cell_pf(const UvwArgs<T> &a, const PrefetchArgs &pf) {
     constexpr int TC = TILE_CELLS;
     const TileBlock<UVW_PF_BLOCK> tb(pf);
@@ -418,7 +430,7 @@ __device__ __forceinline__ void uvw_cell_pf(const UvwArgs<T> &a, const PrefetchA
     const bool lead = tb.lead;
     __shared__ int4 s_rng;
     if (lead) fetch_ranges_async(&s_rng, pf.desc + tp);
-    if (c < a.nC) uvw_cell(a, c);
+    if (c < a.nC) uvw_cell<T, WF>(a, c);
     if (lead) {
         const int64_t L = a.ldg;
         const void *const cellSrc[20] = {a.u, a.v, a.w, a.visC, a.su, a.sv_, a.sw, a.au, a.av, a.aw,
@@ -428,7 +440,11 @@ __device__ __forceinline__ void uvw_cell_pf(const UvwArgs<T> &a, const PrefetchA
 #pragma unroll
         for (int i = 0; i < 19; i++) cellBytes[i] = TC * (int) sizeof(T);
         cellBytes[19] = TC * (int) sizeof(typename UvwReal<T>::V4);
-        prefetch_tile<20>(pf, tp, ranges_ready(&s_rng), a.fg, (int) sizeof(typename UvwReal<T>::V4),
+        const int4 r = ranges_ready(&s_rng);
+        // the face scalars that are set: the carried values' sources and rlencos
+        prefetch_faces(a.carry, r, 4);
+        prefetch_faces(a.rlencos, r, 8);
+        prefetch_tile<20>(pf, tp, r, a.fg, (int) sizeof(typename UvwReal<T>::V4),
                           (const T *) a.massFlux, cellSrc, cellBytes);
     }
 }
@@ -439,20 +455,22 @@ __device__ __forceinline__ void uvw_cell_pf(const UvwArgs<T> &a, const PrefetchA
 // selected once per incidence instead of each value.
 __global__ void __launch_bounds__(256, UVW_CELL_MINB) k_uvw_f64(const __grid_constant__ UvwArgs<double> a) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < a.nC) uvw_cell(a, c);
+    if (c < a.nC) uvw_cell<double, 0>(a, c);
 }
+template <int WF>
 __global__ void __launch_bounds__(UVW_PF_BLOCK, UVW_CELL_MINB *TILE_CELLS / UVW_PF_BLOCK) k_uvw_f64_pf(const __grid_constant__ UvwArgs<double> a,
                                                                           PrefetchArgs pf) {
-    uvw_cell_pf(a, pf);
+    uvw_cell_pf<double, WF>(a, pf);
 }
 // The reference's T = float instantiation.
 __global__ void __launch_bounds__(256, UVW_CELL_MINB) k_uvw_f32ref(const __grid_constant__ UvwArgs<float> a) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < a.nC) uvw_cell(a, c);
+    if (c < a.nC) uvw_cell<float, 0>(a, c);
 }
+template <int WF>
 __global__ void __launch_bounds__(UVW_PF_BLOCK, UVW_CELL_MINB *TILE_CELLS / UVW_PF_BLOCK) k_uvw_f32ref_pf(const __grid_constant__ UvwArgs<float> a,
                                                                              PrefetchArgs pf) {
-    uvw_cell_pf(a, pf);
+    uvw_cell_pf<float, WF>(a, pf);
 }
 
 // ---------------------------------------------------------------------------

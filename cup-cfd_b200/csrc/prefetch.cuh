@@ -81,6 +81,14 @@ __device__ __forceinline__ void warp_partial_store(double l, int c, double *part
         part[(size_t) ((c >> 5) % (TILE_CELLS / 32)) * (gridDim.x / TileBlock<B>::P) + c / TILE_CELLS] = l;
 }
 
+// Prefetches face scalars of `size` bytes (may be null) over a tile's owned
+// faces {.z, .w}, in whole 16-byte units inside that range.
+__device__ __forceinline__ void prefetch_faces(const void *p, const int4 &d, int size) {
+    const uintptr_t from = (reinterpret_cast<uintptr_t>(p) + (size_t) d.z * size + 15) & ~(uintptr_t) 15;
+    const uintptr_t to = (reinterpret_cast<uintptr_t>(p) + (size_t) d.w * size) & ~(uintptr_t) 15;
+    if (p && to > from) bulk_prefetch_l2(reinterpret_cast<const void *>(from), (unsigned) (to - from));
+}
+
 // Prefetches a tile's ranges: its entries, its owned faces' records (fgSize
 // bytes each) and gface values (widened to whole 16-byte units inside the
 // array), and, when the tile is whole, the cell arrays (cellBytes per tile).

@@ -66,6 +66,7 @@ struct CellList {
     __device__ __forceinline__ void load(int k0, int2 (&en)[W]) const {
         load_entries(e, k0, w, en);
     }
+    __device__ __forceinline__ int2 at(int k) const { return ld_entry(e + 32 * k); }  // k < w
 };
 template <>
 struct CellList<-6> {
@@ -99,6 +100,7 @@ struct CellList<-6> {
             en[j] = b;
         }
     }
+    __device__ __forceinline__ int2 at(int k) const { return advance(__ldg(e + k)); }
     __device__ __forceinline__ int2 advance(int2 b) const {
         return make_int2(b.x + 2 * d, b.y >= 0 ? b.y + d : b.y - d);
     }

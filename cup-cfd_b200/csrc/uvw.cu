@@ -139,20 +139,20 @@ int run_face_loop(cupcfd_gpu_mesh *m, T gammaBlend, T small, const T *u, const T
                       a16(su) && a16(sv) && a16(sw) && a16(au) && a16(av) && a16(aw) && a16(grads) &&
                       a16(massFlux) && !prefetch_disabled();
     if (pfOk) {
+        // the run form of the lists where the mesh has it
+        const bool runs = m->fullWidth == 6 && m->sell.runs;
         PrefetchArgs pf;
-        pf.desc = (const TileDesc *) m->tileDesc;
-        pf.inc = m->sell.inc;
-        pf.runHead = nullptr;
+        pf.desc = (const TileDesc *) (runs ? m->tileDescRuns : m->tileDesc);
+        pf.inc = runs ? (const int2 *) m->sell.runs : m->sell.inc;
+        pf.runHead = runs ? m->sell.runHead : nullptr;
         pf.nC = m->nC;
         pf.nF = m->nF;
         pf.nTiles = m->nTiles;
-        if constexpr (F64) {
-            pf.dist = prefetch_wave(m->device, (const void *) k_uvw_f64_pf);
-            k_uvw_f64_pf<<<grid_for(m->nC, TILE_CELLS) * (TILE_CELLS / UVW_PF_BLOCK), UVW_PF_BLOCK, 0, st>>>(a, pf);
-        } else {
-            pf.dist = prefetch_wave(m->device, (const void *) k_uvw_f32ref_pf);
-            k_uvw_f32ref_pf<<<grid_for(m->nC, TILE_CELLS) * (TILE_CELLS / UVW_PF_BLOCK), UVW_PF_BLOCK, 0, st>>>(a, pf);
-        }
+        void (*kern)(UvwArgs<T>, PrefetchArgs);
+        if constexpr (F64) kern = runs ? k_uvw_f64_pf<-6> : k_uvw_f64_pf<0>;
+        else kern = runs ? k_uvw_f32ref_pf<-6> : k_uvw_f32ref_pf<0>;
+        pf.dist = prefetch_wave(m->device, (const void *) kern);
+        kern<<<m->nTiles * (TILE_CELLS / UVW_PF_BLOCK), UVW_PF_BLOCK, 0, st>>>(a, pf);
     } else {
         if constexpr (F64)
             k_uvw_f64<<<grid_for(m->nC, BT), BT, 0, st>>>(a);
