@@ -201,10 +201,6 @@ __device__ __forceinline__ void stage16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned) __cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
-__device__ __forceinline__ void stage8(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned) __cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
 __device__ __forceinline__ void stage4(void *dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned) __cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -217,6 +213,11 @@ __device__ __forceinline__ void stage_wait(int left) {
     else if (left == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
     else asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
+// Used where a cell's arithmetic and values fill the registers (the forward+
+// mass adjoint); kernels with room for more warps are as fast or faster
+// without, FP64 ones included (forward 818 against 604 us at 256^3), and so
+// are full lists, whose scattered gathers the L1 it would take serves (FP32
+// step on a permuted 192^3 mesh 557-577 us against 430).
 // The first two faces stay in registers: on a row of cells they are the x
 // faces, whose values sit in L1 already (staging them too: 0.55 ms against
 // 0.48 for the forward+mass adjoint at 256^3; staging only the last two 0.60).

@@ -31,7 +31,7 @@ __device__ __forceinline__ void block_sum_store(double v, double *out) {
 
 // Per-cell body of the FP64 fused forward (exact reference arithmetic).
 // Returns this cell's loss contribution (0 when gface is null).
-template <int CH, int WF = 0>
+template <int CH, int PIPE = 0, int WF = 0>
 __device__ __forceinline__ double fwd_cell_f64(int c, const SellView &sv, const double4 *__restrict__ fg,
                                                const double *__restrict__ phi, const double *__restrict__ phiB,
                                                const double *__restrict__ vol, const double *__restrict__ st,
@@ -42,9 +42,10 @@ __device__ __forceinline__ double fwd_cell_f64(int c, const SellView &sv, const 
     double phic = phi[c];
     double r0 = st[c], u0 = st[ldc + c], v0 = st[2 * ldc + c], w0 = st[3 * ldc + c];
     double ax = 0.0, ay = 0.0, az = 0.0, lsum = 0.0;
+    int2 en[CH];
+    if (PIPE) e.load(0, en);
     for (int k0 = 0; k0 < w; k0 += CH) {
-        int2 en[CH];
-        e.load(k0, en);
+        if (!PIPE) e.load(k0, en);
         double4 G[CH];
         double pv[CH], so[CH][4], gf[CH];
 #pragma unroll
@@ -60,6 +61,8 @@ __device__ __forceinline__ double fwd_cell_f64(int c, const SellView &sv, const 
                 gf[j] = gface ? __ldg(gface + f) : 0.0;
             }
         }
+        int2 nx[CH];
+        if (PIPE) e.load(k0 + CH, nx);
 #pragma unroll
         for (int j = 0; j < CH; j++) {
             int code = en[j].x;
@@ -84,6 +87,7 @@ __device__ __forceinline__ double fwd_cell_f64(int c, const SellView &sv, const 
             }
             ax = da(ax, dm(phif, G[j].x)); ay = da(ay, dm(phif, G[j].y)); az = da(az, dm(phif, G[j].z));
         }
+        if (PIPE) next_entries<PIPE>(e, k0 + CH, en, nx);
     }
     double V = vol[c];
     double fact = dvd(1.0, V);
@@ -93,7 +97,7 @@ __device__ __forceinline__ double fwd_cell_f64(int c, const SellView &sv, const 
 }
 
 // Per-cell body of the FP32 fused forward; state as float4 {rho, u, v, w}.
-template <int CH, int WF = 0>
+template <int CH, int PIPE = 0, int WF = 0>
 __device__ __forceinline__ double fwd_cell_f32(int c, const SellView &sv, const float4 *__restrict__ fg,
                                                const float *__restrict__ phi, const float *__restrict__ phiB,
                                                const double *__restrict__ vol, const float4 *__restrict__ st,
@@ -106,9 +110,10 @@ __device__ __forceinline__ double fwd_cell_f32(int c, const SellView &sv, const 
     Acc2x2 axy;  // (gx, gy) packed, gz alone
     Acc2 az;
     double lsum = 0.0;
+    int2 en[CH];
+    if (PIPE) e.load(0, en);
     for (int k0 = 0; k0 < w; k0 += CH) {
-        int2 en[CH];
-        e.load(k0, en);
+        if (!PIPE) e.load(k0, en);
         float4 G[CH], so[CH];
         float pv[CH], gf[CH];
 #pragma unroll
@@ -123,6 +128,8 @@ __device__ __forceinline__ double fwd_cell_f32(int c, const SellView &sv, const 
                 gf[j] = gface ? __ldg(gface + f) : 0.f;
             }
         }
+        int2 nx[CH];
+        if (PIPE) e.load(k0 + CH, nx);
 #pragma unroll
         for (int j = 0; j < CH; j++) {
             int code = en[j].x;
@@ -145,6 +152,7 @@ __device__ __forceinline__ double fwd_cell_f32(int c, const SellView &sv, const 
             axy.add_prod(make_float2(phif, phif), make_float2(G[j].x, G[j].y));
             az.add_prod(phif, G[j].z);
         }
+        if (PIPE) next_entries<PIPE>(e, k0 + CH, en, nx);
     }
     double V = vol[c];
     double fact = 1.0 / V;
@@ -580,75 +588,6 @@ __device__ __forceinline__ void adj_cell_f32(int c, const SellView &sv, const fl
     }
     if (doG) phibar[c] = pb.value_f();
     if (doM) stbar[c] = make_float4(rb.value_f(), uvb.xf(), uvb.yf(), wb.value_f());
-}
-
-// The gradient part of adj_cell_f32 for six-entry lists, with the faces past
-// the first CUPCFD_GADJ_STAGE_FROM gathered into shared memory (cp.async)
-// before the first ones' arithmetic; the same sums in the same order.
-#ifndef CUPCFD_GADJ_STAGE_FROM
-#define CUPCFD_GADJ_STAGE_FROM 2
-#endif
-template <int BLOCK>
-struct GadjStage {
-    static constexpr int N = 6 - CUPCFD_GADJ_STAGE_FROM;
-    float4 G[N][BLOCK];
-    float g[N][3][BLOCK];
-};
-template <int ALT, int BLOCK>
-__device__ __forceinline__ void gadj_cell_staged(int c, const CellList<-6> &e, GadjStage<BLOCK> &sh,
-                                                 const float4 *__restrict__ fg, const float *__restrict__ g, float hscale,
-                                                 float *__restrict__ phibar, float *__restrict__ phibBar, int64_t ldc) {
-    constexpr int N = 6, D = CUPCFD_GADJ_STAGE_FROM;
-    const int t = threadIdx.x;
-    int code[N], other[N];  // ALT: the face itself in place of the code
-    if (ALT) {
-        e.template load_alternating<ALT>(code, other);
-    } else {
-        int2 en[N];
-        e.load(0, en);
-#pragma unroll
-        for (int j = 0; j < N; j++) { code[j] = en[j].x; other[j] = en[j].y; }
-    }
-#pragma unroll
-    for (int j = D; j < N; j++) {
-        const int o = other[j];
-        stage16(&sh.G[j - D][t], fg + (ALT ? code[j] : code[j] >> 1));
-        if (ALT > (j < 2 ? 1 : 0) || o >= 0) {
-            stage4(&sh.g[j - D][0][t], g + o);
-            stage4(&sh.g[j - D][1][t], g + ldc + o);
-            stage4(&sh.g[j - D][2][t], g + 2 * ldc + o);
-        }
-        if ((j - D) % 2 == 1) stage_commit();
-    }
-    const float hx = hscale * __ldg(g + c), hy = hscale * __ldg(g + ldc + c), hz = hscale * __ldg(g + 2 * ldc + c);
-    float4 G[D + 1];
-    float go[D + 1][3];
-#pragma unroll
-    for (int j = 0; j < D; j++) {
-        const int o = other[j];
-        G[j] = __ldg(fg + (ALT ? code[j] : code[j] >> 1));
-        if (ALT > (j < 2 ? 1 : 0) || o >= 0) {
-            go[j][0] = __ldg(g + o); go[j][1] = __ldg(g + ldc + o); go[j][2] = __ldg(g + 2 * ldc + o);
-        }
-    }
-    Acc2 pb;
-    auto add = [&](int j, const float4 &G, float g0, float g1, float g2) {
-        if (ALT < (j < 2 ? 2 : 1) && other[j] < 0) {
-            phibBar[-1 - other[j]] = fmaf(hx, G.x, fmaf(hy, G.y, hz * G.z));
-            return;
-        }
-        const FaceW fw = face_weights(G.w, ALT ? j % 2 == 0 : code[j] & 1);
-        const float sx = fmaf(hscale, g0, hx), sy = fmaf(hscale, g1, hy), sz = fmaf(hscale, g2, hz);
-        pb.add_prod(fw.wc, fmaf(sx, G.x, fmaf(sy, G.y, sz * G.z)));
-    };
-#pragma unroll
-    for (int j = 0; j < D; j++) add(j, G[j], go[j][0], go[j][1], go[j][2]);
-#pragma unroll
-    for (int j = D; j < N; j++) {
-        if ((j - D) % 2 == 0) stage_wait((N - j) / 2 - 1);
-        add(j, sh.G[j - D][t], sh.g[j - D][0][t], sh.g[j - D][1][t], sh.g[j - D][2][t]);
-    }
-    phibar[c] = pb.value_f();
 }
 
 __global__ void __launch_bounds__(256, CUPCFD_MINB_ADJ_F64) k_adj_f64(int nC, SellView sv, const double4 *__restrict__ fg,

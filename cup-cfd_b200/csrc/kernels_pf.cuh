@@ -28,6 +28,33 @@ template <int WF> constexpr int PF_BLOCK_MADJ_F64 = 128;
 template <int WF> constexpr int PF_BLOCK_GRAD = 128;
 template <int WF> constexpr int PF_BLOCK_GRAD_ADJ = 128;
 
+// Entries per chunk, whether the next chunk's entries load during the current
+// chunk's arithmetic, and the tiles' worth of blocks per SM the registers
+// allow. In run form the entries come from one cache line, so one face at a
+// time with the next entry ahead leaves registers for more warps, which
+// counts for more: FP32 forward at 256^3 382 us at 1 / ahead / 6 (455 at
+// 3 / no / 4, 410 at 1 / ahead / 5, 424 at 1 / ahead / 7), FP32 adjoint 471 at
+// 1 / ahead / 4 (493 at 2 / no / 4, 544 at 1 / ahead / 5), FP64 forward 604 at
+// 1 / ahead / 4 (748 at 2 / no / 3; 1 / no / 4 613; five and six tiles spill),
+// gradient adjoint 237 at 1 / ahead / 7 and 8 (247 at 2 / ahead / 6; gathered
+// into shared memory like the forward+mass adjoint 240, and 848 against 841
+// us a step under the power limit). On full lists more values in flight per
+// thread count for more: FP64 adjoint of a permuted 96^3 mesh 83 us at 2 / 2
+// against 87 at 1 / 4.
+template <int WF> constexpr int PF_CHUNK_FWD = WF == -6 ? 1 : 3;
+template <int WF> constexpr int PF_PIPE_FWD = WF == -6;
+template <int WF> constexpr int PF_MINB_FWD = WF == -6 ? 6 : 4;
+template <int WF> constexpr int PF_CHUNK_ADJ = WF == -6 ? 1 : 2;
+template <int WF> constexpr int PF_PIPE_ADJ = WF == -6;
+constexpr int PF_MINB_ADJ = 4;
+template <int WF> constexpr int PF_CHUNK_FWD_F64 = WF == -6 ? 1 : 2;
+template <int WF> constexpr int PF_PIPE_FWD_F64 = WF == -6;
+template <int WF> constexpr int PF_MINB_FWD_F64 = WF == -6 ? 4 : 3;
+template <int WF> constexpr int PF_CHUNK_ADJ_F64 = WF == -6 ? 1 : 2;
+template <int WF> constexpr int PF_MINB_ADJ_F64 = WF == -6 ? 4 : 2;
+template <int WF> constexpr int PF_CHUNK_GADJ = WF == -6 ? 1 : 2;
+template <int WF> constexpr int PF_MINB_GADJ = WF == -6 ? 7 : 6;
+
 // Entries per chunk of the gradient kernels, and the tiles' worth of blocks
 // per SM the registers allow. At 128^3 (112^3 permuted for the correction),
 // all in 128-thread blocks: one FP64 gradient 56 us at 2 / 4 (3 / 4 60, 1 / 6
@@ -64,7 +91,7 @@ constexpr int PF_CHUNK_GRAD_ADJ = 3, PF_MINB_GRAD_ADJ = 3;
 // 0.503-0.533 in 256-thread blocks, FP32 adjoint 0.518-0.529 against
 // 0.543-0.583, FP64 forward 0.698-0.704 against 0.707-0.717.
 template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_FWD<WF>, CUPCFD_MINB_F32 *TILE_CELLS / PF_BLOCK_FWD<WF>)
+__global__ void __launch_bounds__(PF_BLOCK_FWD<WF>, PF_MINB_FWD<WF> *TILE_CELLS / PF_BLOCK_FWD<WF>)
     k_fwd_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ phi,
                  const float *__restrict__ phiB, const double *__restrict__ vol, const float4 *__restrict__ st,
                  const float *__restrict__ gface, float *__restrict__ g, float *__restrict__ mflux,
@@ -77,13 +104,13 @@ __global__ void __launch_bounds__(PF_BLOCK_FWD<WF>, CUPCFD_MINB_F32 *TILE_CELLS 
     const int cellBytes[3] = {T * 4, T * 16, T * 8};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     double l = 0.0;
-    if (c < nC) l = fwd_cell_f32<CUPCFD_FWD_CHUNK, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, ldc);
+    if (c < nC) l = fwd_cell_f32<PF_CHUNK_FWD<WF>, PF_PIPE_FWD<WF>, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, ldc);
     if (tb.lead) prefetch_tile<3>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
     if (lossPart) warp_partial_store<PF_BLOCK_FWD<WF>>(l, c, lossPart);
 }
 
 template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_ADJ<WF>, CUPCFD_MINB_F32 *TILE_CELLS / PF_BLOCK_ADJ<WF>)
+__global__ void __launch_bounds__(PF_BLOCK_ADJ<WF>, PF_MINB_ADJ *TILE_CELLS / PF_BLOCK_ADJ<WF>)
     k_adj_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ g, float hscale,
                  const float4 *__restrict__ st, const float *__restrict__ gface, float *__restrict__ phibar,
                  float *__restrict__ phibBar, float4 *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
@@ -94,14 +121,14 @@ __global__ void __launch_bounds__(PF_BLOCK_ADJ<WF>, CUPCFD_MINB_F32 *TILE_CELLS 
     const void *const cellSrc[4] = {g, g + ldc, g + 2 * ldc, st};
     const int cellBytes[4] = {T * 4, T * 4, T * 4, T * 16};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
-    if (c < nC) adj_cell_f32<false, CUPCFD_ADJ_CHUNK, 0, WF>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
+    if (c < nC) adj_cell_f32<false, PF_CHUNK_ADJ<WF>, PF_PIPE_ADJ<WF>, WF>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
     if (tb.lead) prefetch_tile<4>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, gface, cellSrc, cellBytes);
 }
 
 // FP64 forward (fwd_cell_f64, exact reference arithmetic) with the same L2
 // prefetch; the state's four component blocks are prefetched one by one.
 template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_FWD_F64<WF>, CUPCFD_MINB_FWD_F64 *TILE_CELLS / PF_BLOCK_FWD_F64<WF>)
+__global__ void __launch_bounds__(PF_BLOCK_FWD_F64<WF>, PF_MINB_FWD_F64<WF> *TILE_CELLS / PF_BLOCK_FWD_F64<WF>)
     k_fwd_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ phi,
                  const double *__restrict__ phiB, const double *__restrict__ vol, const double *__restrict__ st,
                  const double *__restrict__ gface, double *__restrict__ g, double *__restrict__ mflux,
@@ -114,14 +141,14 @@ __global__ void __launch_bounds__(PF_BLOCK_FWD_F64<WF>, CUPCFD_MINB_FWD_F64 *TIL
     const int cellBytes[6] = {T * 8, T * 8, T * 8, T * 8, T * 8, T * 8};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     double l = 0.0;
-    if (c < nC) l = fwd_cell_f64<CUPCFD_FWD_CHUNK_F64, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, ldc);
+    if (c < nC) l = fwd_cell_f64<PF_CHUNK_FWD_F64<WF>, PF_PIPE_FWD_F64<WF>, WF>(c, sv, fg, phi, phiB, vol, st, gface, g, mflux, ldc);
     if (tb.lead) prefetch_tile<6>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
     if (lossPart) warp_partial_store<PF_BLOCK_FWD_F64<WF>>(l, c, lossPart);
 }
 
 // FP64 adjoint (adj_cell_f64) with the same L2 prefetch.
 template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, CUPCFD_MINB_ADJ_F64 *TILE_CELLS / PF_BLOCK_ADJ_F64<WF>)
+__global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, PF_MINB_ADJ_F64<WF> *TILE_CELLS / PF_BLOCK_ADJ_F64<WF>)
     k_adj_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ g, double hscale,
                  const double *__restrict__ st, const double *__restrict__ gface, double *__restrict__ phibar,
                  double *__restrict__ phibBar, double *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
@@ -132,7 +159,7 @@ __global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, CUPCFD_MINB_ADJ_F64 *TIL
     const void *const cellSrc[7] = {g, g + ldc, g + 2 * ldc, st, st + ldc, st + 2 * ldc, st + 3 * ldc};
     const int cellBytes[7] = {T * 8, T * 8, T * 8, T * 8, T * 8, T * 8, T * 8};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
-    if (c < nC) adj_cell_f64<false, CUPCFD_ADJ_CHUNK_F64, WF>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
+    if (c < nC) adj_cell_f64<false, PF_CHUNK_ADJ_F64<WF>, WF>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
     if (tb.lead) prefetch_tile<7>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
 }
 
@@ -193,20 +220,10 @@ __global__ void __launch_bounds__(PF_BLOCK_FWD_MADJ<WF>, CUPCFD_MINB_FWD_MADJ *T
 
 // Gradient part of the adjoint only (adj_cell_f32 without the mass part):
 // phibar and phibBar. The next chunk's entries load during the current
-// chunk's arithmetic (CUPCFD_GADJ_PIPE) within the 40 registers that six
-// resident blocks per SM leave (CUPCFD_MINB_GADJ): chosen by measurement.
-// On lists in run form it stages the gradients and face records of four faces
-// (gadj_cell_staged, 7 KB a block) in 64-thread blocks: 0.237-0.249 ms against
-// 0.278 at 256^3 (256-thread blocks 0.250, five tiles an SM 0.255-0.269, eight
-// 0.314), 1.14 GB of DRAM traffic against 1.86.
-#ifndef CUPCFD_GADJ_PIPE
-#define CUPCFD_GADJ_PIPE 1
-#endif
-#ifndef CUPCFD_MINB_GADJ
-#define CUPCFD_MINB_GADJ 6
-#endif
+// chunk's arithmetic. 0.278 ms at 256^3 on full lists (1.86 GB of DRAM
+// traffic), 0.237 in run form (1.14 GB).
 template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_GADJ<WF>, CUPCFD_MINB_GADJ *TILE_CELLS / PF_BLOCK_GADJ<WF>)
+__global__ void __launch_bounds__(PF_BLOCK_GADJ<WF>, PF_MINB_GADJ<WF> *TILE_CELLS / PF_BLOCK_GADJ<WF>)
     k_gadj_f32_pf(int nC, SellView sv, const float4 *__restrict__ fg, const float *__restrict__ g, float hscale,
                   float *__restrict__ phibar, float *__restrict__ phibBar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
@@ -216,17 +233,8 @@ __global__ void __launch_bounds__(PF_BLOCK_GADJ<WF>, CUPCFD_MINB_GADJ *TILE_CELL
     const void *const cellSrc[3] = {g, g + ldc, g + 2 * ldc};
     const int cellBytes[3] = {T * 4, T * 4, T * 4};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
-    if (c < nC) {
-        if constexpr (WF == -6) {
-            __shared__ GadjStage<PF_BLOCK_GADJ<WF>> stage;
-            const CellList<WF> e(sv, c);
-            if (e.alternating == 2) gadj_cell_staged<2>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
-            else if (e.alternating == 1) gadj_cell_staged<1>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
-            else gadj_cell_staged<0>(c, e, stage, fg, g, hscale, phibar, phibBar, ldc);
-        } else
-            adj_cell_f32<false, CUPCFD_ADJ_CHUNK, CUPCFD_GADJ_PIPE, WF>(c, sv, fg, g, hscale, nullptr, nullptr, phibar,
-                                                                    phibBar, nullptr, ldc);
-    }
+    if (c < nC)
+        adj_cell_f32<false, PF_CHUNK_GADJ<WF>, 1, WF>(c, sv, fg, g, hscale, nullptr, nullptr, phibar, phibBar, nullptr, ldc);
     if (tb.lead) prefetch_tile<3>(pf, tb.tp, ranges_ready(&s_rng), fg, 16, (const float *) nullptr, cellSrc, cellBytes);
 }
 
@@ -252,7 +260,7 @@ __global__ void __launch_bounds__(PF_BLOCK_MADJ<WF>, CUPCFD_MINB_F32 *TILE_CELLS
 
 // The mass-flux part of the adjoint only, FP64 (adj_cell_f64 with hscale 0).
 template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, CUPCFD_MINB_ADJ_F64 *TILE_CELLS / PF_BLOCK_MADJ_F64<WF>)
+__global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, PF_MINB_ADJ_F64<WF> *TILE_CELLS / PF_BLOCK_MADJ_F64<WF>)
     k_madj_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ st,
                   const double *__restrict__ gface, double *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
@@ -263,7 +271,7 @@ __global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, CUPCFD_MINB_ADJ_F64 *TI
     const int cellBytes[4] = {T * 8, T * 8, T * 8, T * 8};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     if (c < nC)
-        adj_cell_f64<false, CUPCFD_ADJ_CHUNK_F64, WF>(c, sv, fg, nullptr, 0.0, st, gface, nullptr, nullptr, stbar, ldc);
+        adj_cell_f64<false, PF_CHUNK_ADJ_F64<WF>, WF>(c, sv, fg, nullptr, 0.0, st, gface, nullptr, nullptr, stbar, ldc);
     if (tb.lead) prefetch_tile<4>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
 }
 
