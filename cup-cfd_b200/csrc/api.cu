@@ -609,14 +609,6 @@ extern "C" int cupcfd_gpu_dev_adjoint(cupcfd_gpu_mesh *m, int32_t precision, con
     return CUPCFD_E_SUCCESS;
 }
 
-namespace {
-// Above this many tiles the loss reduction runs on the mesh's second stream,
-// beside the gradient adjoint; below, the events that tie the streams cost
-// more than the reduction itself: 14.4 us a call against 16.3 at 128 tiles
-// (32^3 cells), 18.6 against 15.1 at 432 (48^3).
-constexpr unsigned LOSS_BESIDE_TILES = 148;
-}  // namespace
-
 extern "C" int cupcfd_gpu_dev_forward_adjoint(cupcfd_gpu_mesh *m, int32_t precision, const void *phi, const void *phiB,
                                               const void *state, const void *gface, void *grad, void *massFlux,
                                               void *phiBar, void *phiBBar, void *stateBar, double *loss, void *stream) {
@@ -650,27 +642,24 @@ extern "C" int cupcfd_gpu_dev_forward_adjoint(cupcfd_gpu_mesh *m, int32_t precis
         }
         // the FP64 loss reduction (one block) runs on the mesh's second stream
         // beside the gradient adjoint, which does not need it; the caller's
-        // stream waits for both
-        const bool beside = grid > LOSS_BESIDE_TILES;
-        cudaStream_t so = st;
-        if (beside) {
-            so = m->outStream;
-            CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[0], st));
-            CG_CHECK_CUDA(cudaStreamWaitEvent(so, m->pipeEv[0], 0));
-        }
+        // stream waits for both (on one stream: 16.4 us a call against 13.5 at
+        // 24^3, 18.6 against 15.1 at 48^3)
+        cudaStream_t so = m->outStream;
+        CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[0], st));
+        CG_CHECK_CUDA(cudaStreamWaitEvent(so, m->pipeEv[0], 0));
         {
             KTIMER("k_reduce_partials", so);
             k_reduce_partials<WPT><<<1, 1024, 0, so>>>((int) grid, part, lp);
             CG_LAUNCHED();
         }
-        if (beside) CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[1], so));
+        CG_CHECK_CUDA(cudaEventRecord(m->pipeEv[1], so));
         {
             KTIMER("k_gadj_f32_pf", st);
             CG_LAUNCH_PF(m, k_gadj_f32_pf, PF_BLOCK_GADJ, st, m->nC, sell(m), m->fg32, (const float *) grad, 2.f,
                          (float *) phiBar, (float *) phiBBar, m->nC, pfg);
             CG_LAUNCHED();
         }
-        if (beside) CG_CHECK_CUDA(cudaStreamWaitEvent(st, m->pipeEv[1], 0));
+        CG_CHECK_CUDA(cudaStreamWaitEvent(st, m->pipeEv[1], 0));
         return CUPCFD_E_SUCCESS;
     }
     CG_TRY(cupcfd_gpu_dev_forward(m, precision, phi, phiB, state, gface, grad, massFlux, lp, stream));
