@@ -168,6 +168,8 @@ SIGNATURES = {
 def lib():
     """The loaded library (built from csrc/ with nvcc if the .so is missing)."""
     global _lib
+    if _lib is not None:  # set once, complete
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
@@ -219,12 +221,17 @@ def check(rc):
 
 
 def _p(a):
+    """The address of a tensor or host array as a plain integer (what the
+    signatures' void pointers take; a ctypes object per argument cost a small
+    device call 2 us of 14)."""
     if a is None:
         return None
-    if hasattr(a, "data_ptr"):
-        return C.c_void_p(a.data_ptr())
-    assert a.flags["C_CONTIGUOUS"], "host arrays must be C-contiguous"
-    return C.c_void_p(a.ctypes.data)
+    try:
+        return a.data_ptr()
+    except AttributeError:
+        pass
+    assert a.flags.c_contiguous, "host arrays must be C-contiguous"
+    return a.__array_interface__["data"][0]
 
 
 def _vec(a, real_size=8):
@@ -233,20 +240,21 @@ def _vec(a, real_size=8):
     EuclideanVector layout: k = 4 for double gives a 32-byte stride)."""
     if a is None:
         return Vec3View(None, 3 * real_size, 0)
-    assert a.flags["C_CONTIGUOUS"]
+    assert a.flags.c_contiguous
     if a.ndim == 2 and a.shape[1] == 3:
-        return Vec3View(a.ctypes.data, 3 * real_size, 0)
+        return Vec3View(_p(a), 3 * real_size, 0)
     if a.ndim == 2 and a.shape[1] == 4:
-        return Vec3View(a.ctypes.data, 4 * real_size, real_size)
+        return Vec3View(_p(a), 4 * real_size, real_size)
     raise ValueError("vector arrays must be (n,3) packed or (n,4) with a leading pad slot")
 
 
 def _stream(s):
     if s is None:
         return None
-    if hasattr(s, "cuda_stream"):
-        return C.c_void_p(s.cuda_stream)
-    return C.c_void_p(int(s))
+    try:
+        return s.cuda_stream
+    except AttributeError:
+        return int(s)
 
 
 # ---------------------------------------------------------------------------
