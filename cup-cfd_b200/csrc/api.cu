@@ -537,6 +537,15 @@ const char *launch_fwd_f64(const cupcfd_gpu_mesh *m, const void *phi, const void
 }
 }  // namespace
 
+namespace {
+// Up to this many tiles the loss's last pass sums each tile's eight partials
+// itself instead of after a pass of its own: forward with loss 10.3 us against
+// 13.5 at 54 tiles (24^3 cells), 14.4 against 18.5 at 1,024 (64^3), 33.0
+// against 35.1 at 3,456 (96^3), 49.3 either way at 5,488, 97 against 95 (FP64)
+// at 8,192 (128^3), where one block reads half a megabyte.
+constexpr unsigned LOSS_DIRECT_TILES = 4096;
+}  // namespace
+
 extern "C" int cupcfd_gpu_dev_forward(cupcfd_gpu_mesh *m, int32_t precision, const void *phi, const void *phiB,
                                       const void *state, const void *gface, void *grad, void *massFlux, double *loss,
                                       void *stream) {
@@ -560,15 +569,18 @@ extern "C" int cupcfd_gpu_dev_forward(cupcfd_gpu_mesh *m, int32_t precision, con
         CG_LAUNCHED();
     }
     if (loss) {
-        // per-warp partials: each tile's value first (many blocks), then the
-        // fixed-order sum over tiles; the same bits as per-tile partials
-        if (group > 1) {
+        // per-warp partials: where there are many, each tile's value first (many
+        // blocks), then the fixed-order sum over tiles; the same bits as per-tile
+        // partials and as summing each tile's eight in the last pass
+        const bool direct = group > 1 && grid <= LOSS_DIRECT_TILES;
+        if (group > 1 && !direct) {
             KTIMER("k_group_partials", st);
             k_group_partials<TILE_CELLS / 32><<<grid_for(grid, BLK), BLK, 0, st>>>((int) grid, part);
             CG_LAUNCHED();
         }
         KTIMER("k_reduce_partials", st);
-        k_reduce_partials<<<1, 1024, 0, st>>>((int) grid, part, loss);
+        if (direct) k_reduce_partials<TILE_CELLS / 32><<<1, 1024, 0, st>>>((int) grid, part, loss);
+        else k_reduce_partials<<<1, 1024, 0, st>>>((int) grid, part, loss);
         CG_LAUNCHED();
     }
     return CUPCFD_E_SUCCESS;
@@ -1304,12 +1316,14 @@ extern "C" int cupcfd_gpu_dev_forward_noalloc(cupcfd_gpu_mesh *m, int32_t precis
     g_launches.fetch_add(1, std::memory_order_relaxed);
     if (cudaGetLastError() != cudaSuccess) return CUPCFD_E_ERROR;
     if (loss) {
-        if (group > 1) {
+        const bool direct = group > 1 && grid <= LOSS_DIRECT_TILES;  // as cupcfd_gpu_dev_forward
+        if (group > 1 && !direct) {
             k_group_partials<TILE_CELLS / 32><<<grid_for(grid, BLK), BLK, 0, st>>>((int) grid, part);
             g_launches.fetch_add(1, std::memory_order_relaxed);
             if (cudaGetLastError() != cudaSuccess) return CUPCFD_E_ERROR;
         }
-        k_reduce_partials<<<1, 1024, 0, st>>>((int) grid, part, loss);
+        if (direct) k_reduce_partials<TILE_CELLS / 32><<<1, 1024, 0, st>>>((int) grid, part, loss);
+        else k_reduce_partials<<<1, 1024, 0, st>>>((int) grid, part, loss);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (cudaGetLastError() != cudaSuccess) return CUPCFD_E_ERROR;
     }
