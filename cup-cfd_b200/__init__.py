@@ -223,15 +223,14 @@ def check(rc):
 def _p(a):
     """The address of a tensor or host array as a plain integer (what the
     signatures' void pointers take; a ctypes object per argument cost a small
-    device call 2 us of 14)."""
+    device call 2 us of 14). Host arrays first: a caught AttributeError for each
+    cost the drop-in calls 10 us of 425."""
     if a is None:
         return None
-    try:
+    if not isinstance(a, np.ndarray):
         return a.data_ptr()
-    except AttributeError:
-        pass
     assert a.flags.c_contiguous, "host arrays must be C-contiguous"
-    return a.__array_interface__["data"][0]
+    return a.ctypes.data
 
 
 def _vec(a, real_size=8):
