@@ -406,3 +406,15 @@ def test_gradient_and_general_adjoints_prefetch_equals_plain(cg, gpu, kind, dims
         outs.append(o + [pb, pbb, sb])
     for a, b in zip(*outs):
         assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dims", [(128, 128, 64),    # 4,096 tiles: the last summed by one pass
+                                  (129, 128, 64)])   # 4,128: folded by many blocks first
+def test_forward_loss_is_the_pipelines(cg, gpu, dims):
+    """The forward's loss adds the tiles' partials in one order whether one
+    pass or two take them: the bits of the forward+adjoint call's loss, which
+    takes one at every size."""
+    import torch
+    mesh = cg.Mesh.structgen(*dims, order=cg.ORDER_OWNER)
+    fields = _fields(torch, mesh, 31)
+    _assert_same(_run(cg, torch, mesh, *fields, offset=False), _run_pipeline(cg, torch, mesh, *fields, offset=False))
