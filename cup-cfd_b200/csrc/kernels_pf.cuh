@@ -39,8 +39,11 @@ template <int WF> constexpr int PF_BLOCK_GRAD_ADJ = 128;
 // gradient adjoint 237 at 1 / ahead / 7 and 8 (247 at 2 / ahead / 6; gathered
 // into shared memory like the forward+mass adjoint 240, and 848 against 841
 // us a step under the power limit). On full lists more values in flight per
-// thread count for more: FP64 adjoint of a permuted 96^3 mesh 83 us at 2 / 2
-// against 87 at 1 / 4.
+// thread count for more: FP64 adjoint of a permuted 96^3 mesh 78 us at 3 / 2
+// (83 at 2 / 2, 87 at 1 / 4, 125 spilling at 6 / 2), 128^3 154 against 163 at
+// 2 / 2, 160^3 316 against 334, 48^3 17 either way; both adjoints in Morton
+// order at 128^3 153 against 160. The FP64 forward stays at 2 / 3: 2 / 2 takes
+// 68 against 72 at 96^3, but 15 against 13 at 48^3 and the same from 128^3 on.
 template <int WF> constexpr int PF_CHUNK_FWD = WF == -6 ? 1 : 3;
 template <int WF> constexpr int PF_PIPE_FWD = WF == -6;
 template <int WF> constexpr int PF_MINB_FWD = WF == -6 ? 6 : 4;
@@ -50,7 +53,7 @@ constexpr int PF_MINB_ADJ = 4;
 template <int WF> constexpr int PF_CHUNK_FWD_F64 = WF == -6 ? 1 : 2;
 template <int WF> constexpr int PF_PIPE_FWD_F64 = WF == -6;
 template <int WF> constexpr int PF_MINB_FWD_F64 = WF == -6 ? 4 : 3;
-template <int WF> constexpr int PF_CHUNK_ADJ_F64 = WF == -6 ? 1 : 2;
+template <int WF> constexpr int PF_CHUNK_ADJ_F64 = WF == -6 ? 1 : WF == 6 ? 3 : 2;
 template <int WF> constexpr int PF_MINB_ADJ_F64 = WF == -6 ? 4 : 2;
 template <int WF> constexpr int PF_CHUNK_GADJ = WF == -6 ? 1 : 2;
 template <int WF> constexpr int PF_MINB_GADJ = WF == -6 ? 7 : 6;

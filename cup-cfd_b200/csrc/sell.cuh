@@ -64,6 +64,7 @@ struct CellList {
     }
     template <int W>
     __device__ __forceinline__ void load(int k0, int2 (&en)[W]) const {
+        static_assert(!WF || 6 % W == 0, "the six-entry forms test for no padding: chunks divide six");
         load_entries(e, k0, w, en);
     }
     __device__ __forceinline__ int2 at(int k) const { return ld_entry(e + 32 * k); }  // k < w
@@ -84,6 +85,7 @@ struct CellList<-6> {
     }
     template <int W>
     __device__ __forceinline__ void load(int k0, int2 (&en)[W]) const {
+        static_assert(6 % W == 0, "no padding: chunks divide six");
 #pragma unroll
         for (int j = 0; j < W; j++) {
             int2 b = make_int2(-1, -1);
