@@ -9,8 +9,14 @@
 // powers of two, though, all its values are multiples of one unit u in the
 // last place, and adding v rounds the real number acc + v to the nearest
 // multiple: acc / u grows by the integer nearest to v / u, whatever acc is.
-// Those integers are added in parallel, exactly, and the partial sums are the
-// chain's own values. Only a tie (v / u an integer and a half) looks at acc:
+// Those integers are added in parallel, and the partial sums are the chain's
+// own values, provided no addition on the way rounds. A stretch of consecutive
+// integers adds up to the difference of two partial sums, both between the
+// same powers of two (2^52 and 2^53 units), so to less than 2^52: exact. Sums
+// of every second or fourth thread or warp, as a butterfly of exchanges forms
+// them, have no such bound (values that rise through one thread's share and
+// fall through the next pass 2^53) and serve only where the integers' sizes
+// add up to less than 2^51. Only a tie (v / u an integer and a half) looks at acc:
 // it goes to the even neighbour, which the parities of the integers since the
 // tie before tell. Where a partial sum leaves the interval between the powers
 // of two (or a value is not finite, or too large), the additions up to there
@@ -189,16 +195,17 @@ __global__ void __launch_bounds__(OS_T) k_ordered_sum(const __grid_constant__ Or
                     sum = __dadd_rn(sum, step[k]);
                     size = __dadd_rn(size, fabs(step[k]));
                 }
-                double warpSum = sum;
+                double at = sum;  // with the warp's threads before: consecutive, so exact up to where the scan ends
 #pragma unroll
-                for (int d = 16; d > 0; d >>= 1) {
-                    warpSum = __dadd_rn(warpSum, __shfl_xor_sync(0xffffffffu, warpSum, d));
+                for (int d = 1; d < 32; d <<= 1) {
+                    const double p = __shfl_up_sync(0xffffffffu, at, d);
+                    if (lane >= d) at = __dadd_rn(at, p);
                     size = __dadd_rn(size, __shfl_xor_sync(0xffffffffu, size, d));
                 }
                 const unsigned odds = __ballot_sync(0xffffffffu, odd);  // of the warp's threads
                 turnSums ^= 1;
-                if (lane == 0) {
-                    warpSums[turnSums][wid] = make_double2(warpSum, size);
+                if (lane == 31) {
+                    warpSums[turnSums][wid] = make_double2(at, size);
                     warpOdd[turnSums][wid] = __popc(odds) & 1;
                 }
                 if (t == 0) {
@@ -259,17 +266,15 @@ __global__ void __launch_bounds__(OS_T) k_ordered_sum(const __grid_constant__ Or
                 }
                 // Else the partial sums themselves, up to the first that
                 // leaves the interval, tie, or value too large or not finite.
-                double at = sum;
+                double warps = w.x;  // with the warps before
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const double p = __shfl_up_sync(0xffffffffu, at, d);
-                    if (lane >= d) at = __dadd_rn(at, p);
+                for (int d = 1; d < NW; d <<= 1) {
+                    const double p = __shfl_up_sync(0xffffffffu, warps, d);
+                    if (lane >= d) warps = __dadd_rn(warps, p);
                 }
-                double warpsBefore = lane < wid ? w.x : 0.0;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) warpsBefore = __dadd_rn(warpsBefore, __shfl_xor_sync(0xffffffffu, warpsBefore, d));
+                warps = __shfl_sync(0xffffffffu, warps, max(wid - 1, 0));
                 at = __shfl_up_sync(0xffffffffu, at, 1);
-                at = __dadd_rn(__dadd_rn(start, warpsBefore), lane > 0 ? at : 0.0);
+                at = __dadd_rn(wid > 0 ? __dadd_rn(start, warps) : start, lane > 0 ? at : 0.0);
                 int first = OS_B;
 #pragma unroll
                 for (int k = 0; k < OS_E; k++) {

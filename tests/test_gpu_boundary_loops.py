@@ -258,3 +258,44 @@ def test_ordered_sum_rounds_as_the_chain(cg, gpu, kind, n):
             assert same(got, total), (t, got, total)
             if rtype == 2:
                 assert same(acc, want_acc), (t, acc, want_acc)
+
+
+def _swings(group, n, rng, unit):
+    """Values whose running sum rises through `group` of them and falls through the next, inside (1, 2);
+    multiples of unit (0: any; those of an amplitude far above the sum's last place often tie)."""
+    v = np.empty(n)
+    v[0] = at = 1.05
+    for i in range(1, n, group):
+        w = rng.uniform(0.5, 1.5, min(group, n - i))
+        to = (1.05 if at > 1.5 else 1.85) + rng.uniform(0, 0.1)
+        w *= (to - at) / w.sum()
+        v[i:i + group] = np.round(w / unit) * unit if unit else w
+        at += v[i:i + group].sum()
+    return v
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 8200])
+@pytest.mark.parametrize("group", [8, 16, 32, 64, 256, 512, 1024])   # 8: one thread's additions, 256: one warp's
+def test_ordered_sum_of_swinging_values(cg, gpu, group, n):
+    """Totals and region sums of values that swing between two powers of two
+    in step with the threads or warps of the sum, against the chain."""
+    rng = np.random.default_rng(group + n)
+    mesh = cg.Mesh.structgen(40, 41, 42, order=cg.ORDER_OWNER)
+    nB, nF = mesh.nBoundaries, mesh.nFaces
+    face = np.empty(nB, np.int64)
+    bnd = mesh.geometry()["faceBnd"]
+    face[bnd[bnd >= 0]] = np.nonzero(bnd >= 0)[0]
+    chosen = np.sort(rng.choice(nB, n, replace=False))
+    region = np.zeros(nB, np.int32)
+    region[chosen] = 1
+    assert mesh.set_regions([0, 2], np.zeros((2, 3)), np.ones(2), region) == cg.E_SUCCESS
+    for seed in range(40):
+        for t in (np.float64, np.float32):
+            unit = np.finfo(t).eps if seed % 4 < 2 else 0
+            v = ((-1) ** seed * _swings(group, n, np.random.default_rng(seed), unit)).astype(t)
+            mf, acc = np.zeros(nF, t), np.zeros(2, t)
+            mf[face[chosen]] = v
+            rc, got = cg.FluxMassDolfynBoundaryLoop2(mesh, mf, acc)
+            assert rc == cg.E_SUCCESS, cg.last_error()
+            want = np.add.accumulate(v)[-1]   # one addition after another
+            assert got == want and acc[1] == want, (seed, t, got, acc[1], want)
