@@ -1008,13 +1008,6 @@ extern "C" int cupcfd_gpu_mesh_get_info(const cupcfd_gpu_mesh *m, cupcfd_mesh_in
 }
 
 namespace {
-__global__ void k_check_regions(int nB, int nR, const int *__restrict__ br, int *__restrict__ err) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nB && (br[i] < 0 || br[i] >= nR)) atomicOr(err, 1);
-}
-}  // namespace
-
-namespace {
 
 // faces of listed boundaries
 __global__ void k_list_faces(int n, const int *__restrict__ id, const int *__restrict__ faceRef,
@@ -1077,32 +1070,26 @@ extern "C" int cupcfd_gpu_mesh_set_regions(cupcfd_gpu_mesh *m, int32_t nR, const
     for (int r = 0; r < nR; r++)
         CG_RETURN_IF(type[r] < CUPCFD_RTYPE_DEFAULT || type[r] > CUPCFD_RTYPE_WALL, CUPCFD_E_CONFIG_INVALID_VALUE,
                      "set_regions: unknown region type");
+    // every id before anything changes: after a refused call the mesh has the regions it had
+    bool bad = false;
+    for (int b = 0; b < nB; b++) bad |= (uint32_t) bndRegion[b] >= (uint32_t) nR;
+    CG_RETURN_IF(bad, CUPCFD_E_INVALID_INDEX, "set_regions: a boundary's region id is out of range");
     CG_TRY(make_device_current(m->device));
     cudaStream_t st = m->stream;
     if (nR > m->nR) {
-        CG_TRY(m->alloc(&m->regionType, (size_t) nR));
-        CG_TRY(m->alloc(&m->regionUVW, 3 * (size_t) nR));
-        CG_TRY(m->alloc(&m->regionDen, (size_t) nR));
-        CG_TRY(m->alloc(&m->regionSplvl, (size_t) nR));
+        int *rt;
+        double *ru, *rd, *rs;
+        CG_TRY(m->alloc(&rt, (size_t) nR));
+        CG_TRY(m->alloc(&ru, 3 * (size_t) nR));
+        CG_TRY(m->alloc(&rd, (size_t) nR));
+        CG_TRY(m->alloc(&rs, (size_t) nR));
+        m->regionType = rt; m->regionUVW = ru; m->regionDen = rd; m->regionSplvl = rs;
     }
     CG_CHECK_CUDA(cudaMemsetAsync(m->regionSplvl, 0, sizeof(double) * nR, st));
     CG_CHECK_CUDA(cudaMemcpyAsync(m->regionType, type, sizeof(int) * nR, cudaMemcpyHostToDevice, st));
     CG_CHECK_CUDA(cudaMemcpyAsync(m->regionUVW, uvw, sizeof(double) * 3 * nR, cudaMemcpyHostToDevice, st));
     CG_CHECK_CUDA(cudaMemcpyAsync(m->regionDen, den, sizeof(double) * nR, cudaMemcpyHostToDevice, st));
-    if (nB > 0) {
-        int *err;
-        void *ev;
-        CG_TRY(m->scratchBuf(0, sizeof(int), &ev));
-        err = (int *) ev;
-        CG_CHECK_CUDA(cudaMemcpyAsync(m->bndRegion, bndRegion, sizeof(int) * nB, cudaMemcpyHostToDevice, st));
-        CG_CHECK_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-        k_check_regions<<<grid_for(nB, 256), 256, 0, st>>>(nB, nR, m->bndRegion, err);
-        CG_LAUNCHED();
-        int h = 0;
-        CG_CHECK_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CG_CHECK_CUDA(cudaStreamSynchronize(st));
-        CG_RETURN_IF(h != 0, CUPCFD_E_INVALID_INDEX, "set_regions: a boundary's region id is out of range");
-    }
+    if (nB > 0) CG_CHECK_CUDA(cudaMemcpyAsync(m->bndRegion, bndRegion, sizeof(int) * nB, cudaMemcpyHostToDevice, st));
     CG_CHECK_CUDA(cudaStreamSynchronize(st));
     CG_TRY(build_bnd_lists(m, nR, type, bndRegion));
     m->nR = nR;

@@ -299,3 +299,22 @@ def test_ordered_sum_of_swinging_values(cg, gpu, group, n):
             assert rc == cg.E_SUCCESS, cg.last_error()
             want = np.add.accumulate(v)[-1]   # one addition after another
             assert got == want and acc[1] == want, (seed, t, got, acc[1], want)
+
+
+@pytest.mark.parametrize("more", [0, 3])
+@pytest.mark.parametrize("wrong", [-1, "nR"])
+def test_refused_regions_leave_the_mesh_as_it_was(cg, gpu, wrong, more):
+    """set_regions with a region id out of range changes nothing: the chain
+    then gives what it gave before (other types, ids and region counts in the
+    refused call)."""
+    m, splvl, mesh, d = _setup(cg, "struct", 2)
+    solve = (1, 0, 1)
+    want = _host_chain(cg, mesh, d, solve)
+    nR = m["nRegions"] + more
+    types = np.resize(np.roll(m["regionType"], 1), nR)
+    ids = np.random.default_rng(5).integers(0, nR, m["nBnd"]).astype(np.int32)
+    ids[m["nBnd"] // 2] = nR if wrong == "nR" else wrong
+    assert mesh.set_regions(types, np.ones((nR, 3)), np.ones(nR), ids) == cg.E_INVALID_INDEX
+    got = _host_chain(cg, mesh, d, solve)
+    for k, x in want.items():
+        assert np.array_equal(got[k], x), k
