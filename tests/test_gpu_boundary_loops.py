@@ -318,3 +318,26 @@ def test_refused_regions_leave_the_mesh_as_it_was(cg, gpu, wrong, more):
     got = _host_chain(cg, mesh, d, solve)
     for k, x in want.items():
         assert np.array_equal(got[k], x), k
+
+
+def test_regions_set_again(cg, gpu):
+    """Loop 2's sums after regions of other counts and types replaced the ones before."""
+    mesh = cg.Mesh.structgen(23, 19, 17, order=cg.ORDER_OWNER)
+    nB, nF = mesh.nBoundaries, mesh.nFaces
+    bnd = mesh.geometry()["faceBnd"]
+    face = np.empty(nB, np.int64)
+    face[bnd[bnd >= 0]] = np.nonzero(bnd >= 0)[0]
+    rng = np.random.default_rng(9)
+    mf = rng.standard_normal(nF)
+    for nR in (2, 7, 3, 300, 1, 5000, 2):
+        types = rng.integers(0, 5, nR).astype(np.int32)
+        types[nR // 2] = 2
+        region = rng.integers(0, nR, nB).astype(np.int32)
+        assert mesh.set_regions(types, np.zeros((nR, 3)), np.ones(nR), region) == cg.E_SUCCESS
+        acc = rng.standard_normal(nR)
+        total, want = 0.0, acc.copy()
+        for b in np.nonzero(types[region] == 2)[0]:
+            total += mf[face[b]]
+            want[region[b]] += mf[face[b]]
+        rc, got = cg.FluxMassDolfynBoundaryLoop2(mesh, mf, acc)
+        assert rc == cg.E_SUCCESS and got == total and np.array_equal(acc, want), nR
