@@ -608,7 +608,9 @@ __global__ void __launch_bounds__(256, CUPCFD_MINB_F32) k_adj_f32(int nC, SellVi
 
 // General gradient adjoint (input gbar = dL/dg, any loss): h_c = gbar_c / V_c
 // (ivol = 1 / V, kept with the mesh: six divisions per cell fewer). FP64
-// arithmetic on T's geometry and fields.
+// arithmetic on T's geometry and fields, with the roundings written out: the
+// plain and the L2-prefetch kernels give the same bits, whatever a compiler
+// would fuse.
 template <bool SIGNED, class T, int CH, int WF>
 __device__ __forceinline__ void grad_adj_cell(int c, const SellView &sv, const typename Vec4<T>::type *__restrict__ fg,
                                               const double *__restrict__ ivol, const T *__restrict__ gbar,
@@ -640,14 +642,15 @@ __device__ __forceinline__ void grad_adj_cell(int c, const SellView &sv, const t
             const int o = en[j].y;
             const bool isN = en[j].x & 1;
             const double Sx = G[j].x, Sy = G[j].y, Sz = G[j].z, lam = G[j].w;
-            const double own = __fma_rn(hz, Sz, __fma_rn(hy, Sy, __dmul_rn(hx, Sx)));
+            const double own = __fma_rn(hz, Sz, __fma_rn(hx, Sx, __dmul_rn(hy, Sy)));
             if (o < 0) {
                 phibBar[-1 - o] = (T) own;
                 continue;
             }
-            const double oth = __dmul_rn(__fma_rn((double) go[j][2], Sz, __fma_rn((double) go[j][1], Sy, __dmul_rn((double) go[j][0], Sx))), io[j]);
+            const double gS = __fma_rn((double) go[j][2], Sz, __fma_rn((double) go[j][0], Sx, __dmul_rn((double) go[j][1], Sy)));
             // d g_P / d phi_f = +S/V_P; d g_N / d phi_f = +S/V_N (reference) or -S/V_N (signed)
-            const double sum = SIGNED ? (isN ? __dsub_rn(oth, own) : __dsub_rn(own, oth)) : __dadd_rn(own, oth);
+            const double oth = __dmul_rn(gS, io[j]);
+            const double sum = SIGNED ? (isN ? __dsub_rn(oth, own) : __dsub_rn(own, oth)) : __fma_rn(gS, io[j], own);
             pb = __fma_rn(isN ? lam : __dsub_rn(1.0, lam), sum, pb);
         }
     }
