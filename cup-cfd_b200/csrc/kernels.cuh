@@ -417,7 +417,7 @@ __device__ __forceinline__ void grad_cell_f32(int c, const SellView &sv, const f
                     float a0 = __fmaf_rn(facn, gN0, __fmul_rn(facp, gP0));
                     float a1 = __fmaf_rn(facn, gN1, __fmul_rn(facp, gP1));
                     float a2 = __fmaf_rn(facn, gN2, __fmul_rn(facp, gP2));
-                    phif = __fadd_rn(phif, __fmaf_rn(a2, d2, __fmaf_rn(a1, d1, __fmul_rn(a0, d0))));
+                    phif = __fadd_rn(phif, __fmaf_rn(a2, d2, __fmaf_rn(a0, d0, __fmul_rn(a1, d1))));
                 }
             }
             if (SIGNED && isN) {

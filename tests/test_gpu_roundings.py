@@ -65,3 +65,68 @@ def test_gradient_adjoint_roundings(cg, gpu, kind, order, f64, sign):
                             stream=torch.cuda.current_stream())
     assert np.array_equal(phi.cpu().numpy(), want)
     assert np.array_equal(phiB.cpu().numpy(), wantB)
+
+
+def f32(q):
+    """The float nearest to a rational, ties to even."""
+    x = np.float32(float(q))
+    return min((np.nextafter(x, np.float32(-np.inf)), x, np.nextafter(x, np.float32(np.inf))),
+               key=lambda y: (abs(Q(float(y)) - q), int(y.view(np.int32)) & 1))
+
+
+def fmaf(a, b, c):
+    return f32(Q(float(a)) * Q(float(b)) + Q(float(c)))
+
+
+class Sum:
+    """A compensated sum of products as the FP32 kernels keep it."""
+    def __init__(self):
+        self.s = self.e = np.float32(0)
+
+    def add(self, a, b):
+        t = self.s + fmaf(a, b, 0)
+        nbp = self.s - t
+        ar = self.s - (t + nbp)
+        self.e = self.e + (ar + fmaf(a, b, nbp))
+        self.s = t
+
+
+@pytest.mark.parametrize("sign", [0, 1])
+@pytest.mark.parametrize("kind,order", MESHES[:2])
+def test_corrected_gradient_roundings_f32(cg, gpu, kind, order, sign):
+    """dev_gradient in FP32 with one non-orthogonal correction: the three
+    products of gradient and distance summed y, x, z by FMAs, then added to
+    the interpolated value."""
+    import torch
+    mesh, geo = _mesh(cg, kind, order)
+    nC, nB = mesh.nCells, mesh.nBoundaries
+    r = np.random.default_rng(2)
+    phi, phiB = r.standard_normal(nC).astype(np.float32), r.standard_normal(nB).astype(np.float32)
+    S, lam, xf, xc = (geo[k].astype(np.float32) for k in ("faceNorm", "faceLambda", "faceCenter", "cellCenter"))
+    fact = 1.0 / geo["cellVolume"]
+    one, grad = np.float32(1), None
+    for _ in range(2):
+        to = np.empty((nC, 3), np.float32)
+        for c in range(nC):
+            sums = [Sum() for _ in range(3)]
+            for f, isN, o in geo["inc"][c]:
+                if o < 0:
+                    phif = phiB[-1 - o]
+                else:
+                    n, p = lam[f], one - lam[f]
+                    N, P = (c, o) if isN else (o, c)
+                    wc, wo = (n, p) if isN else (p, n)
+                    phif = fmaf(wc, phi[c], wo * phi[o])
+                    if grad is not None:
+                        d = [xf[f, k] - fmaf(n, xc[N, k], p * xc[P, k]) for k in range(3)]
+                        a = [fmaf(n, grad[N, k], p * grad[P, k]) for k in range(3)]
+                        phif = phif + fmaf(a[2], d[2], fmaf(a[0], d[0], a[1] * d[1]))
+                for k in range(3):
+                    sums[k].add(-phif if sign and isN else phif, S[f, k])
+            to[c] = [np.float32((float(x.s) + float(x.e)) * fact[c]) for x in sums]
+        grad = to
+    dev = lambda a: torch.from_numpy(a).to(gpu)
+    g = torch.empty(3, nC, device=gpu)
+    cg.dev_gradient(mesh, cg.PREC_F32C, dev(phi), dev(phiB), g, nGradient=2, sign_mode=sign,
+                    stream=torch.cuda.current_stream())
+    assert np.array_equal(g.cpu().numpy().T, grad)
