@@ -264,6 +264,8 @@ __device__ __forceinline__ double fwd_madj_cell_f32(int c, const SellView &sv, c
 // boundary's and every role is known, with 1 past the first two).
 template <int BLOCK>
 struct FwdMadjStage {
+    static_assert(CUPCFD_STAGE_FROM >= 0 && CUPCFD_STAGE_FROM < 6 && CUPCFD_STAGE_FROM % 2 == 0,
+                  "the copies are committed, and waited for, in pairs of faces");
     static constexpr int N = 6 - CUPCFD_STAGE_FROM;
     float4 G[N][BLOCK], so[N][BLOCK];
     float pv[N][BLOCK], gf[N][BLOCK];

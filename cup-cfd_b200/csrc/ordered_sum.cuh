@@ -62,6 +62,9 @@ constexpr int OS_T = CUPCFD_OS_T;  // threads of a block
 constexpr int OS_E = 4096 / OS_T;  // consecutive additions a thread takes
 constexpr int OS_B = OS_T * OS_E;  // additions a block holds at a time
 constexpr int OS_TIES = 16;        // ties a batch may have and still be taken at once
+static_assert(OS_T % 32 == 0 && OS_T <= 1024 && OS_B == 4096 && OS_E % 2 == 0,
+              "whole warps, at most one per lane of a warp; the values in pairs");
+static_assert(CUPCFD_OS_FIRST > 0, "the additions one by one go on");
 
 // The unit of acc's interval between powers of two, and its inverse; false
 // where the scan does not apply (zero, subnormal, not finite, or powers
