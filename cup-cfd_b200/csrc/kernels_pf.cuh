@@ -25,7 +25,7 @@ template <int WF> constexpr int PF_BLOCK_FWD_MADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_GADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_MADJ = 256;
 template <int WF> constexpr int PF_BLOCK_MADJ_F64 = 128;
-template <int WF> constexpr int PF_BLOCK_GRAD = 128;
+template <int WF> constexpr int PF_BLOCK_GRAD = WF == 0 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_GRAD_ADJ = 128;
 
 // Entries per chunk, whether the next chunk's entries load during the current
@@ -44,11 +44,15 @@ template <int WF> constexpr int PF_BLOCK_GRAD_ADJ = 128;
 // 2 / 2, 160^3 316 against 334, 48^3 17 either way; both adjoints in Morton
 // order at 128^3 153 against 160. The FP64 forward stays at 2 / 3: 2 / 2 takes
 // 68 against 72 at 96^3, but 15 against 13 at 48^3 and the same from 128^3 on.
+// Lists of varying width (meshes of merged hexahedra, 6 to 26 faces a cell, at
+// 5,220 / 96,253 / 632,627 cells): FP32 adjoint with the entries ahead 12.6 /
+// 20.8 / 105 us against 14.8 / 20.8 / 112 without (plain kernel 14.7 / 20.8 /
+// 107; three entries 25 / 43 / 206 spilling).
 template <int WF> constexpr int PF_CHUNK_FWD = WF == -6 ? 1 : 3;
 template <int WF> constexpr int PF_PIPE_FWD = WF == -6;
 template <int WF> constexpr int PF_MINB_FWD = WF == -6 ? 6 : 4;
 template <int WF> constexpr int PF_CHUNK_ADJ = WF == -6 ? 1 : 2;
-template <int WF> constexpr int PF_PIPE_ADJ = WF == -6;
+template <int WF> constexpr int PF_PIPE_ADJ = WF != 6;
 constexpr int PF_MINB_ADJ = 4;
 template <int WF> constexpr int PF_CHUNK_FWD_F64 = WF == -6 ? 1 : 2;
 template <int WF> constexpr int PF_PIPE_FWD_F64 = WF == -6;
@@ -68,9 +72,13 @@ template <int WF> constexpr int PF_MINB_GADJ = WF == -6 ? 7 : 6;
 // iteration; on rows in run form 314 at 1 / 3, 333 at 2 / 2, against 527. The
 // general adjoint 3 / 3: with the mass adjoint 154 us, 2 / 4 156, 1 / 4 160,
 // against 241 (its plain kernel took the incidences one by one, with a
-// division each).
-template <bool CORR, int WF> constexpr int PF_CHUNK_GRAD = CORR && WF == -6 ? 1 : 2;
-template <bool CORR, int WF> constexpr int PF_MINB_GRAD = CORR ? (WF == -6 ? 3 : 2) : 4;
+// division each). On lists of varying width (the meshes above) one gradient
+// takes 10.6 / 15.1 / 90 us in FP64 and 8.6 / 12.5 / 61 in FP32 at 4 / 3 in
+// 64-thread blocks, against 12.6 / 16.7 / 96 and 10.6 / 13.8 / 74 at 2 / 4 in
+// 128-thread blocks and 10.5 / 20.1 / 109 and 9.6 / 12.8 / 62 for the plain
+// kernels.
+template <bool CORR, int WF> constexpr int PF_CHUNK_GRAD = CORR ? (WF == -6 ? 1 : 2) : WF == 0 ? 4 : 2;
+template <bool CORR, int WF> constexpr int PF_MINB_GRAD = CORR ? (WF == -6 ? 3 : 2) : WF == 0 ? 3 : 4;
 constexpr int PF_CHUNK_GRAD_ADJ = 3, PF_MINB_GRAD_ADJ = 3;
 
 // ---------------------------------------------------------------------------
