@@ -126,8 +126,25 @@ template <int WF> constexpr auto k_corr_f64_pf = k_grad_pf<double, true, WF>;
 template <int WF> constexpr auto k_corr_f32_pf = k_grad_pf<float, true, WF>;
 template <int WF> constexpr auto k_grad_adj_f64_pf = k_grad_adj_pf<double, WF>;
 template <int WF> constexpr auto k_grad_adj_f32_pf = k_grad_adj_pf<float, WF>;
+template <int WF> constexpr auto k_adj_f64_deep_pf = k_adj_f64_pf<WF, WF != -6>;  // (run form: one form)
+template <int WF> constexpr auto k_adj_f64_warps_pf = k_adj_f64_pf<WF, false>;
 
 inline bool aligned16(const void *p) { return ((uintptr_t) p & 15u) == 0; }
+
+// Whether the FP64 adjoint holds more values per thread (two tiles of blocks an
+// SM) rather than more warps (three to four). On full lists where a warp
+// gathers from many lines, except where the four tiles take one wave and the
+// two two: permuted meshes 56^3 19 us against 21, 100^3 85 / 94, 144^3 233 /
+// 250, numbered at random 96^3 210 / 218; 44^3 12.7 / 10.6, 48^3 14.7 / 12.6,
+// 52^3 17 either way. Generated meshes in Morton order gather from 4 to 5
+// lines: 48^3 11.7 / 10.5, 72^3 31 / 29, 96^3 60 / 61, 128^3 116 / 105, 192^3
+// 417 / 381. On lists of varying width where the two tiles take one wave:
+// merged hexahedra, 5,220 cells 14 / 17, 96,253 37 / 29, 632,627 177 / 181.
+bool adj_f64_deep(const cupcfd_gpu_mesh *m, int sms) {
+    const int wf = list_form(m);
+    if (wf == 0) return m->nTiles <= 2 * sms;
+    return wf == 6 && m->gatherLines >= 7.0 && (m->nTiles <= 2 * sms || m->nTiles > 4 * sms);
+}
 
 // Builds the per-tile ranges the L2-prefetch kernels of both precisions read
 // and the prefetch distance of each kernel; leaves m->tiles false (plain
@@ -140,21 +157,27 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
     TileDesc *desc;
     CG_TRY(m->alloc(&desc, (size_t) m->nTiles));
     m->tileDesc = desc;
-    int *start, *aux;  // aux: [0..2] maxima, [3] order flag
+    int *start, *aux;  // aux: [0..2] maxima, [3] order flag, [4..7] gathered lines and gathers
     CG_TRY(m->alloc(&start, (size_t) m->nTiles + 1));
-    CG_TRY(m->alloc(&aux, 4));
-    CG_CHECK_CUDA(cudaMemsetAsync(aux, 0, 4 * sizeof(int), st));
+    CG_TRY(m->alloc(&aux, 8));
+    CG_CHECK_CUDA(cudaMemsetAsync(aux, 0, 8 * sizeof(int), st));
     k_tile_face_start<<<grid_for(m->nF, BLK), BLK, 0, st>>>(m->nF, m->nTiles, m->faceCells, start, aux + 3);
     CG_LAUNCHED();
     k_tile_desc<<<grid_for(m->nTiles, BLK), BLK, 0, st>>>(m->nTiles, m->sell.nSlices, m->sell.slicePtr, start, desc, aux);
     CG_LAUNCHED();
-    int h[4];
-    CG_CHECK_CUDA(cudaMemcpyAsync(h, aux, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CG_CHECK_CUDA(cudaStreamSynchronize(st));
-    if (h[3] != 0 || h[2] > 255) return CUPCFD_E_SUCCESS;  // faces not by owner tile, or too wide a slice
     int dev = 0, sms = 0;
     CG_CHECK_CUDA(cudaGetDevice(&dev));
     CG_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    k_gather_lines<<<std::min(grid_for((int64_t) m->sell.nSlices * 32, BLK), 8u * sms), BLK, 0, st>>>(
+        m->sell.nSlices, m->sell.slicePtr, m->sell.inc, (unsigned long long *) (aux + 4));
+    CG_LAUNCHED();
+    int h[8];
+    CG_CHECK_CUDA(cudaMemcpyAsync(h, aux, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CG_CHECK_CUDA(cudaStreamSynchronize(st));
+    unsigned long long lines[2];
+    std::memcpy(lines, h + 4, sizeof(lines));
+    m->gatherLines = lines[1] ? (double) lines[0] / (double) lines[1] : 0.0;
+    if (h[3] != 0 || h[2] > 255) return CUPCFD_E_SUCCESS;  // faces not by owner tile, or too wide a slice
     // prefetch one wave of resident blocks ahead (the block that will take
     // this block's place), the best distance measured; each kernel's own
     // wave (the gradient adjoint holds more blocks per SM than the forward:
@@ -166,6 +189,7 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
     m->fullWidth = m->sell.width == 6 && (int64_t) m->nInc == 6 * (int64_t) m->nC &&
                    !(fw && std::strcmp(fw, "0") == 0) ? 6 : 0;
     const int wf = list_form(m);
+    m->adjF64Deep = adj_f64_deep(m, sms);
     if (wf == -6) {
         TileDesc *dr;
         CG_TRY(m->alloc(&dr, (size_t) m->nTiles));
@@ -179,7 +203,7 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
         PF_KERNEL(k_fwd_f32_pf),
         PF_KERNEL(k_adj_f32_pf),
         PF_KERNEL(k_fwd_f64_pf),
-        PF_KERNEL(k_adj_f64_pf),
+        m->adjF64Deep ? PF_KERNEL(k_adj_f64_deep_pf) : PF_KERNEL(k_adj_f64_warps_pf),
         PF_KERNEL(k_fwd_madj_f32_pf),
         PF_KERNEL(k_gadj_f32_pf),
         PF_KERNEL(k_madj_f32_pf),
@@ -599,9 +623,13 @@ extern "C" int cupcfd_gpu_dev_adjoint(cupcfd_gpu_mesh *m, int32_t precision, con
     if (precision == CUPCFD_PREC_F64 && m->tiles && aligned16(grad) && aligned16(state) &&
         aligned16(gface)) {
         kt.set_name("k_adj_f64_pf");
-        CG_LAUNCH_PF(m, k_adj_f64_pf, PF_BLOCK_ADJ_F64, st, m->nC, sell(m), m->fg64, (const double *) grad, 2.0,
-                     (const double *) state, (const double *) gface, (double *) phiBar, (double *) phiBBar,
-                     (double *) stateBar, m->nC, prefetch_args(m, PF_ADJ_F64));
+#define ADJ_PF(K)                                                                                               \
+    CG_LAUNCH_PF(m, K, PF_BLOCK_ADJ_F64, st, m->nC, sell(m), m->fg64, (const double *) grad, 2.0,               \
+                 (const double *) state, (const double *) gface, (double *) phiBar, (double *) phiBBar,         \
+                 (double *) stateBar, m->nC, prefetch_args(m, PF_ADJ_F64))
+        if (m->adjF64Deep) ADJ_PF(k_adj_f64_deep_pf);
+        else ADJ_PF(k_adj_f64_warps_pf);
+#undef ADJ_PF
     } else if (precision == CUPCFD_PREC_F64) {
         kt.set_name("k_adj_f64");
         k_adj_f64<<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, (const double *) grad, 2.0, (const double *) state,

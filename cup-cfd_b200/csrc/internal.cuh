@@ -184,6 +184,8 @@ struct cupcfd_gpu_mesh {
     void *tileDescRuns = nullptr;  // the same with the run form's ranges as the entry ranges
     int nTiles = 0;
     bool tiles = false;
+    double gatherLines = 0.0;     // 128-byte lines a warp's gather of neighbours touches (k_gather_lines)
+    bool adjF64Deep = false;      // form of the FP64 adjoint (adj_f64_deep in api.cu)
     int prefetchDist = 0;         // tiles ahead for the L2 prefetch
     int prefetchWave[16] = {};  // per prefetch kernel (PfKernel in api.cu): one wave of its blocks, in tiles
 

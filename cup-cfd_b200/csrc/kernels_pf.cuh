@@ -20,7 +20,7 @@ namespace cupcfd_gpu {
 template <int WF> constexpr int PF_BLOCK_FWD = 64;
 template <int WF> constexpr int PF_BLOCK_ADJ = 64;
 template <int WF> constexpr int PF_BLOCK_FWD_F64 = 64;
-template <int WF> constexpr int PF_BLOCK_ADJ_F64 = 128;
+template <int WF> constexpr int PF_BLOCK_ADJ_F64 = WF == 0 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_FWD_MADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_GADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_MADJ = 256;
@@ -38,12 +38,9 @@ template <int WF> constexpr int PF_BLOCK_GRAD_ADJ = 128;
 // 1 / ahead / 4 (748 at 2 / no / 3; 1 / no / 4 613; five and six tiles spill),
 // gradient adjoint 237 at 1 / ahead / 7 and 8 (247 at 2 / ahead / 6; gathered
 // into shared memory like the forward+mass adjoint 240, and 848 against 841
-// us a step under the power limit). On full lists more values in flight per
-// thread count for more: FP64 adjoint of a permuted 96^3 mesh 78 us at 3 / 2
-// (83 at 2 / 2, 87 at 1 / 4, 125 spilling at 6 / 2), 128^3 154 against 163 at
-// 2 / 2, 160^3 316 against 334, 48^3 17 either way; both adjoints in Morton
-// order at 128^3 153 against 160. The FP64 forward stays at 2 / 3: 2 / 2 takes
-// 68 against 72 at 96^3, but 15 against 13 at 48^3 and the same from 128^3 on.
+// us a step under the power limit). The FP64 forward stays at 2 / 3 on full
+// lists: 2 / 2 takes 68 against 72 at 96^3, but 15 against 13 at 48^3 and the
+// same from 128^3 on.
 // Lists of varying width (meshes of merged hexahedra, 6 to 26 faces a cell, at
 // 5,220 / 96,253 / 632,627 cells): FP32 adjoint with the entries ahead 12.6 /
 // 20.8 / 105 us against 14.8 / 20.8 / 112 without (plain kernel 14.7 / 20.8 /
@@ -57,8 +54,10 @@ constexpr int PF_MINB_ADJ = 4;
 template <int WF> constexpr int PF_CHUNK_FWD_F64 = WF == -6 ? 1 : 2;
 template <int WF> constexpr int PF_PIPE_FWD_F64 = WF == -6;
 template <int WF> constexpr int PF_MINB_FWD_F64 = WF == -6 ? 4 : 3;
-template <int WF> constexpr int PF_CHUNK_ADJ_F64 = WF == -6 ? 1 : WF == 6 ? 3 : 2;
-template <int WF> constexpr int PF_MINB_ADJ_F64 = WF == -6 ? 4 : 2;
+// The FP64 adjoint in two forms (adj_f64_deep in api.cu chooses): DEEP, more
+// values in flight per thread, and more warps. Its mass part is as DEEP.
+template <int WF, bool DEEP> constexpr int PF_CHUNK_ADJ_F64 = DEEP ? (WF == 6 ? 3 : 2) : 1;
+template <int WF, bool DEEP> constexpr int PF_MINB_ADJ_F64 = DEEP ? 2 : WF == 0 ? 3 : 4;
 template <int WF> constexpr int PF_CHUNK_GADJ = WF == -6 ? 1 : 2;
 template <int WF> constexpr int PF_MINB_GADJ = WF == -6 ? 7 : 6;
 
@@ -158,8 +157,8 @@ __global__ void __launch_bounds__(PF_BLOCK_FWD_F64<WF>, PF_MINB_FWD_F64<WF> *TIL
 }
 
 // FP64 adjoint (adj_cell_f64) with the same L2 prefetch.
-template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, PF_MINB_ADJ_F64<WF> *TILE_CELLS / PF_BLOCK_ADJ_F64<WF>)
+template <int WF, bool DEEP>
+__global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, PF_MINB_ADJ_F64<WF, DEEP> *TILE_CELLS / PF_BLOCK_ADJ_F64<WF>)
     k_adj_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ g, double hscale,
                  const double *__restrict__ st, const double *__restrict__ gface, double *__restrict__ phibar,
                  double *__restrict__ phibBar, double *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, PF_MINB_ADJ_F64<WF> *TIL
     const void *const cellSrc[7] = {g, g + ldc, g + 2 * ldc, st, st + ldc, st + 2 * ldc, st + 3 * ldc};
     const int cellBytes[7] = {T * 8, T * 8, T * 8, T * 8, T * 8, T * 8, T * 8};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
-    if (c < nC) adj_cell_f64<false, PF_CHUNK_ADJ_F64<WF>, WF>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
+    if (c < nC) adj_cell_f64<false, PF_CHUNK_ADJ_F64<WF, DEEP>, WF>(c, sv, fg, g, hscale, st, gface, phibar, phibBar, stbar, ldc);
     if (tb.lead) prefetch_tile<7>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
 }
 
@@ -271,7 +270,7 @@ __global__ void __launch_bounds__(PF_BLOCK_MADJ<WF>, CUPCFD_MINB_F32 *TILE_CELLS
 
 // The mass-flux part of the adjoint only, FP64 (adj_cell_f64 with hscale 0).
 template <int WF>
-__global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, PF_MINB_ADJ_F64<WF> *TILE_CELLS / PF_BLOCK_MADJ_F64<WF>)
+__global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, PF_MINB_ADJ_F64<WF, WF != -6> *TILE_CELLS / PF_BLOCK_MADJ_F64<WF>)
     k_madj_f64_pf(int nC, SellView sv, const double4 *__restrict__ fg, const double *__restrict__ st,
                   const double *__restrict__ gface, double *__restrict__ stbar, int64_t ldc, PrefetchArgs pf) {
     constexpr int T = TILE_CELLS;
@@ -282,7 +281,7 @@ __global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, PF_MINB_ADJ_F64<WF> *TI
     const int cellBytes[4] = {T * 8, T * 8, T * 8, T * 8};
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     if (c < nC)
-        adj_cell_f64<false, PF_CHUNK_ADJ_F64<WF>, WF>(c, sv, fg, nullptr, 0.0, st, gface, nullptr, nullptr, stbar, ldc);
+        adj_cell_f64<false, PF_CHUNK_ADJ_F64<WF, WF != -6>, WF>(c, sv, fg, nullptr, 0.0, st, gface, nullptr, nullptr, stbar, ldc);
     if (tb.lead) prefetch_tile<4>(pf, tb.tp, ranges_ready(&s_rng), fg, 32, gface, cellSrc, cellBytes);
 }
 
@@ -333,6 +332,29 @@ __global__ void __launch_bounds__(PF_BLOCK_GRAD_ADJ<WF>, PF_MINB_GRAD_ADJ *TILE_
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     if (c < nC) grad_adj_cell<false, T, PF_CHUNK_GRAD_ADJ, WF>(c, sv, fg, ivol, gbar, phibar, phibBar, ldc);
     if (tb.lead) prefetch_tile<4>(pf, tb.tp, ranges_ready(&s_rng), fg, 4 * S, (const T *) nullptr, cellSrc, cellBytes);
+}
+
+// The mean number of 128-byte lines of an FP64 cell array that a warp's 32
+// cells gather from for one of their entries: lines[0] lines over lines[1]
+// gathers. 2.2 on generated meshes by rows, 3 to 5 in Morton or RCM order, 7
+// to 10 on irregular meshes in those orders (each cell has its own order of
+// faces), 31 on hexahedra numbered at random (16 on mixed cells).
+__global__ void k_gather_lines(int nSlices, const int *__restrict__ slicePtr, const int2 *__restrict__ inc,
+                               unsigned long long *__restrict__ lines) {
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    unsigned n = 0, gathers = 0;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nSlices; s += warps)
+        for (int k = slicePtr[s]; k < slicePtr[s + 1]; k += 32) {
+            const int o = inc[k + lane].y, line = o >= 0 ? o >> 4 : -1;
+            const unsigned same = __match_any_sync(0xffffffffu, line);
+            const unsigned first = __ballot_sync(0xffffffffu, line >= 0 && __ffs((int) same) - 1 == lane);
+            n += __popc(first);
+            gathers += first != 0;
+        }
+    if (lane == 0) {
+        atomicAdd(lines, (unsigned long long) n);
+        atomicAdd(lines + 1, (unsigned long long) gathers);
+    }
 }
 
 // Largest |c - neighbour| over the incidence lists (the numbering's bandwidth).

@@ -418,3 +418,41 @@ def test_forward_loss_is_the_pipelines(cg, gpu, dims):
     mesh = cg.Mesh.structgen(*dims, order=cg.ORDER_OWNER)
     fields = _fields(torch, mesh, 31)
     _assert_same(_run(cg, torch, mesh, *fields, offset=False), _run_pipeline(cg, torch, mesh, *fields, offset=False))
+
+
+@pytest.mark.parametrize("kind,dims,order", [("structgen", (20, 18, 17), "ORDER_MORTON"),   # gathers from few lines
+                                             ("jittered", (20, 18, 17), "ORDER_MORTON"),    # from many: values in flight
+                                             ("jittered", (45, 45, 45), "ORDER_RCM"),       # 356 tiles: one wave of four an SM
+                                             ("jittered", (56, 54, 53), "ORDER_MORTON"),    # 627: more
+                                             ("poly", (20, 18, 17), "ORDER_MORTON"),
+                                             ("poly", (62, 60, 61), "ORDER_MORTON")])       # over 296 tiles
+def test_fp64_adjoint_forms_equal_the_plain_kernel(cg, gpu, kind, dims, order):
+    """Each form of the FP64 adjoint's L2-prefetch kernel, as the mesh's lists
+    and size choose it, with the plain kernel's bits."""
+    import torch
+    if kind == "poly":
+        import oracle as O
+        mesh = cg.Mesh.from_arrays(O.merge_cells(O.jitter(*dims, 0.25, seed=5, permute=True), 0.3, 11, max_cells=6),
+                                   order=getattr(cg, order))
+        assert mesh.full_width == 0
+    else:
+        mesh = _mesh(cg, kind, dims, order)
+    nC, nB = mesh.nCells, mesh.nBoundaries
+    st, gface = (x.double() for x in _fields(torch, mesh, 37)[2:])
+    st = st.t().contiguous()
+    grad = torch.randn(3 * nC + 1, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda", dtype=torch.float64)
+    outs = []
+    for name, g in (("k_adj_f64_pf", grad[:-1].clone()), ("k_adj_f64", grad[1:])):
+        if name == "k_adj_f64":
+            g.copy_(grad[:-1].clone())   # the same values, 8 bytes past a 16-byte boundary
+        o = [torch.full(n, float("nan"), dtype=torch.float64, device="cuda") for n in ((nC,), (nB,), (4, nC))]
+        cg.timing_read()
+        cg.timing_enable(True)
+        try:
+            cg.dev_adjoint(mesh, cg.PREC_F64, g, st, gface, *o, stream=torch.cuda.current_stream())
+            assert set(cg.timing_read()) == {name}
+        finally:
+            cg.timing_enable(False)
+        outs.append(o)
+    for a, b in zip(*outs):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
