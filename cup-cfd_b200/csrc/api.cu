@@ -121,7 +121,8 @@ class KernelTimer {
 
 // the kernel templates of more than the list form, by that alone
 template <int WF> constexpr auto k_grad_f64_pf = k_grad_pf<double, false, WF>;
-template <int WF> constexpr auto k_grad_f32_pf = k_grad_pf<float, false, WF>;
+template <int WF> constexpr auto k_grad_f64_deep_pf = k_grad_pf<double, false, WF, WF == 0>;  // (full lists: one form)
+template <int WF> constexpr auto k_grad_f32_pf = k_grad_pf<float, false, WF, WF == 0>;
 template <int WF> constexpr auto k_corr_f64_pf = k_grad_pf<double, true, WF>;
 template <int WF> constexpr auto k_corr_f32_pf = k_grad_pf<float, true, WF>;
 template <int WF> constexpr auto k_grad_adj_f64_pf = k_grad_adj_pf<double, WF>;
@@ -131,19 +132,25 @@ template <int WF> constexpr auto k_adj_f64_warps_pf = k_adj_f64_pf<WF, false>;
 
 inline bool aligned16(const void *p) { return ((uintptr_t) p & 15u) == 0; }
 
-// Whether the FP64 adjoint holds more values per thread (two tiles of blocks an
-// SM) rather than more warps (three to four). On full lists where a warp
-// gathers from many lines, except where the four tiles take one wave and the
-// two two: permuted meshes 56^3 19 us against 21, 100^3 85 / 94, 144^3 233 /
-// 250, numbered at random 96^3 210 / 218; 44^3 12.7 / 10.6, 48^3 14.7 / 12.6,
-// 52^3 17 either way. Generated meshes in Morton order gather from 4 to 5
-// lines: 48^3 11.7 / 10.5, 72^3 31 / 29, 96^3 60 / 61, 128^3 116 / 105, 192^3
-// 417 / 381. On lists of varying width where the two tiles take one wave:
-// merged hexahedra, 5,220 cells 14 / 17, 96,253 37 / 29, 632,627 177 / 181.
-bool adj_f64_deep(const cupcfd_gpu_mesh *m, int sms) {
-    const int wf = list_form(m);
-    if (wf == 0) return m->nTiles <= 2 * sms;
-    return wf == 6 && m->gatherLines >= 7.0 && (m->nTiles <= 2 * sms || m->nTiles > 4 * sms);
+// Which forms of the FP64 adjoint and of the FP64 gradient suit the mesh: DEEP
+// ones hold more values per thread, in fewer tiles' worth of blocks an SM.
+// Adjoint on full lists (two tiles an SM against four): DEEP where a warp
+// gathers from many lines, except where the four take one wave and the two
+// two: permuted meshes 56^3 19 us against 21, 100^3 85 / 94, 144^3 233 / 250,
+// numbered at random 96^3 210 / 218; 44^3 12.7 / 10.6, 48^3 14.7 / 12.6, 52^3
+// 17 either way. Generated meshes in Morton order gather from 4 to 5 lines:
+// 48^3 11.7 / 10.5, 72^3 31 / 29, 96^3 60 / 61, 128^3 116 / 105, 192^3 417 / 381.
+// On lists of varying width both run at the same rate, so DEEP unless its waves
+// hold more tiles than the other's, the last ones' empty places counted. Merged
+// hexahedra of 5,220 / 96,253 / 136,991 / 412,485 / 632,627 cells (21 / 376 /
+// 536 / 1,612 / 2,471 tiles on 148 SMs): adjoint (two against three an SM) 14.5
+// / 37 / 42 / 121 / 177 us against 18 / 31 / 54 / 132 / 181, gradient (three
+// against four) 10.6 / 15.1 / 24.6 / 66 / 90 against 12.6 / 16.7 / 18.9 / 69 / 96.
+void forms_setup(cupcfd_gpu_mesh *m, int sms) {
+    const int wf = list_form(m), n = m->nTiles;
+    auto places = [&](int tiles) { return (n + tiles * sms - 1) / (tiles * sms) * (int64_t) tiles; };
+    m->adjF64Deep = wf == 0 ? places(2) <= places(3) : wf == 6 && m->gatherLines >= 7.0 && (n <= 2 * sms || n > 4 * sms);
+    m->gradF64Deep = wf == 0 && places(3) <= places(4);
 }
 
 // Builds the per-tile ranges the L2-prefetch kernels of both precisions read
@@ -189,7 +196,7 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
     m->fullWidth = m->sell.width == 6 && (int64_t) m->nInc == 6 * (int64_t) m->nC &&
                    !(fw && std::strcmp(fw, "0") == 0) ? 6 : 0;
     const int wf = list_form(m);
-    m->adjF64Deep = adj_f64_deep(m, sms);
+    forms_setup(m, sms);
     if (wf == -6) {
         TileDesc *dr;
         CG_TRY(m->alloc(&dr, (size_t) m->nTiles));
@@ -208,7 +215,7 @@ int tiles_setup(cupcfd_gpu_mesh *m, cudaStream_t st) {
         PF_KERNEL(k_gadj_f32_pf),
         PF_KERNEL(k_madj_f32_pf),
         PF_KERNEL(k_madj_f64_pf),
-        PF_KERNEL(k_grad_f64_pf),
+        m->gradF64Deep ? PF_KERNEL(k_grad_f64_deep_pf) : PF_KERNEL(k_grad_f64_pf),
         PF_KERNEL(k_grad_f32_pf),
         PF_KERNEL(k_corr_f64_pf),
         PF_KERNEL(k_corr_f32_pf),
@@ -309,6 +316,7 @@ int launch_grad_once(cupcfd_gpu_mesh *m, int precision, bool corr, bool sgn, con
                  (const T *) prev, (T *) grad, (T *) gcopy, ldc, prefetch_args(m, W))
         if (precision == CUPCFD_PREC_F64) {
             if (corr) GRAD_PF(double, fg64, fc64, cc64, k_corr_f64_pf, PF_BLOCK_GRAD, PF_CORR_F64);
+            else if (m->gradF64Deep) GRAD_PF(double, fg64, fc64, cc64, k_grad_f64_deep_pf, PF_BLOCK_GRAD, PF_GRAD_F64);
             else GRAD_PF(double, fg64, fc64, cc64, k_grad_f64_pf, PF_BLOCK_GRAD, PF_GRAD_F64);
         } else {
             if (corr) GRAD_PF(float, fg32, fc32, cc32, k_corr_f32_pf, PF_BLOCK_GRAD, PF_CORR_F32);

@@ -185,7 +185,7 @@ struct cupcfd_gpu_mesh {
     int nTiles = 0;
     bool tiles = false;
     double gatherLines = 0.0;     // 128-byte lines a warp's gather of neighbours touches (k_gather_lines)
-    bool adjF64Deep = false;      // form of the FP64 adjoint (adj_f64_deep in api.cu)
+    bool adjF64Deep = false, gradF64Deep = false;  // forms of the FP64 adjoint and gradient (forms_setup in api.cu)
     int prefetchDist = 0;         // tiles ahead for the L2 prefetch
     int prefetchWave[16] = {};  // per prefetch kernel (PfKernel in api.cu): one wave of its blocks, in tiles
 

@@ -18,9 +18,9 @@ namespace cupcfd_gpu {
 // adjoint in 256), 425 in 128, 431 in 256, 464 in 512; FP64 forward and
 // adjoint at 96^3 70 / 92 in 64, 72 / 87 in 128, 74 / 90 in 256.
 template <int WF> constexpr int PF_BLOCK_FWD = 64;
-template <int WF> constexpr int PF_BLOCK_ADJ = 64;
+template <int WF> constexpr int PF_BLOCK_ADJ = WF == 0 ? 256 : 64;
 template <int WF> constexpr int PF_BLOCK_FWD_F64 = 64;
-template <int WF> constexpr int PF_BLOCK_ADJ_F64 = WF == 0 ? 64 : 128;
+template <int WF> constexpr int PF_BLOCK_ADJ_F64 = 128;
 template <int WF> constexpr int PF_BLOCK_FWD_MADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_GADJ = WF == -6 ? 64 : 128;
 template <int WF> constexpr int PF_BLOCK_MADJ = 256;
@@ -42,9 +42,10 @@ template <int WF> constexpr int PF_BLOCK_GRAD_ADJ = 128;
 // lists: 2 / 2 takes 68 against 72 at 96^3, but 15 against 13 at 48^3 and the
 // same from 128^3 on.
 // Lists of varying width (meshes of merged hexahedra, 6 to 26 faces a cell, at
-// 5,220 / 96,253 / 632,627 cells): FP32 adjoint with the entries ahead 12.6 /
-// 20.8 / 105 us against 14.8 / 20.8 / 112 without (plain kernel 14.7 / 20.8 /
-// 107; three entries 25 / 43 / 206 spilling).
+// 5,220 / 136,991 / 632,627 cells): FP32 adjoint with the entries ahead in
+// 256-thread blocks 14.5 / 24.9 / 103 us, in 64-thread blocks 12.6 / 26.9 /
+// 106, without the entries ahead 14.7 / 26.9 / 112, plain kernel 14.7 / 25.0 /
+// 108 (three entries spill: 206).
 template <int WF> constexpr int PF_CHUNK_FWD = WF == -6 ? 1 : 3;
 template <int WF> constexpr int PF_PIPE_FWD = WF == -6;
 template <int WF> constexpr int PF_MINB_FWD = WF == -6 ? 6 : 4;
@@ -54,7 +55,7 @@ constexpr int PF_MINB_ADJ = 4;
 template <int WF> constexpr int PF_CHUNK_FWD_F64 = WF == -6 ? 1 : 2;
 template <int WF> constexpr int PF_PIPE_FWD_F64 = WF == -6;
 template <int WF> constexpr int PF_MINB_FWD_F64 = WF == -6 ? 4 : 3;
-// The FP64 adjoint in two forms (adj_f64_deep in api.cu chooses): DEEP, more
+// The FP64 adjoint in two forms (forms_setup in api.cu chooses): DEEP, more
 // values in flight per thread, and more warps. Its mass part is as DEEP.
 template <int WF, bool DEEP> constexpr int PF_CHUNK_ADJ_F64 = DEEP ? (WF == 6 ? 3 : 2) : 1;
 template <int WF, bool DEEP> constexpr int PF_MINB_ADJ_F64 = DEEP ? 2 : WF == 0 ? 3 : 4;
@@ -71,13 +72,13 @@ template <int WF> constexpr int PF_MINB_GADJ = WF == -6 ? 7 : 6;
 // iteration; on rows in run form 314 at 1 / 3, 333 at 2 / 2, against 527. The
 // general adjoint 3 / 3: with the mass adjoint 154 us, 2 / 4 156, 1 / 4 160,
 // against 241 (its plain kernel took the incidences one by one, with a
-// division each). On lists of varying width (the meshes above) one gradient
-// takes 10.6 / 15.1 / 90 us in FP64 and 8.6 / 12.5 / 61 in FP32 at 4 / 3 in
-// 64-thread blocks, against 12.6 / 16.7 / 96 and 10.6 / 13.8 / 74 at 2 / 4 in
-// 128-thread blocks and 10.5 / 20.1 / 109 and 9.6 / 12.8 / 62 for the plain
-// kernels.
-template <bool CORR, int WF> constexpr int PF_CHUNK_GRAD = CORR ? (WF == -6 ? 1 : 2) : WF == 0 ? 4 : 2;
-template <bool CORR, int WF> constexpr int PF_MINB_GRAD = CORR ? (WF == -6 ? 3 : 2) : WF == 0 ? 3 : 4;
+// division each). On lists of varying width (the meshes above) one FP32 gradient
+// takes 8.6 / 15.7 / 61 us DEEP, 4 / 3 in 64-thread blocks, against 10.6 / 15.9
+// / 74 at 2 / 4 in 128-thread blocks and 9.6 / 16.7 / 62 for the plain kernel;
+// the FP64 one 10.6 / 24.6 / 90 DEEP, 12.6 / 18.9 / 96 at 2 / 4, 10.5 / 22.3 /
+// 109 plain (forms_setup in api.cu chooses).
+template <bool CORR, int WF, bool DEEP> constexpr int PF_CHUNK_GRAD = CORR ? (WF == -6 ? 1 : 2) : DEEP ? 4 : 2;
+template <bool CORR, int WF, bool DEEP> constexpr int PF_MINB_GRAD = CORR ? (WF == -6 ? 3 : 2) : DEEP ? 3 : 4;
 constexpr int PF_CHUNK_GRAD_ADJ = 3, PF_MINB_GRAD_ADJ = 3;
 
 // ---------------------------------------------------------------------------
@@ -288,8 +289,8 @@ __global__ void __launch_bounds__(PF_BLOCK_MADJ_F64<WF>, PF_MINB_ADJ_F64<WF, WF 
 // The gradient by itself (grad_cell_*, reference sign), with the L2 prefetch;
 // CORR: an iteration with the non-orthogonal correction, which reads the
 // previous iterate go and the cells' and faces' centres as well.
-template <class T, bool CORR, int WF>
-__global__ void __launch_bounds__(PF_BLOCK_GRAD<WF>, PF_MINB_GRAD<CORR, WF> *TILE_CELLS / PF_BLOCK_GRAD<WF>)
+template <class T, bool CORR, int WF, bool DEEP = false>
+__global__ void __launch_bounds__(PF_BLOCK_GRAD<WF>, PF_MINB_GRAD<CORR, WF, DEEP> *TILE_CELLS / PF_BLOCK_GRAD<WF>)
     k_grad_pf(int nC, SellView sv, const typename Vec4<T>::type *__restrict__ fg, const typename Vec4<T>::type *__restrict__ fc,
               const typename Vec4<T>::type *__restrict__ cc, const T *__restrict__ phi, const T *__restrict__ phiB,
               const double *__restrict__ vol, const T *__restrict__ go, T *__restrict__ g, T *__restrict__ gcopy, int64_t ldc,
@@ -301,9 +302,9 @@ __global__ void __launch_bounds__(PF_BLOCK_GRAD<WF>, PF_MINB_GRAD<CORR, WF> *TIL
     if (tb.lead) fetch_ranges_async(&s_rng, pf.desc + tb.tp);
     if (c < nC) {
         if constexpr (S == 8)
-            grad_cell_f64<CORR, false, PF_CHUNK_GRAD<CORR, WF>, WF>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
+            grad_cell_f64<CORR, false, PF_CHUNK_GRAD<CORR, WF, DEEP>, WF>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
         else
-            grad_cell_f32<CORR, false, PF_CHUNK_GRAD<CORR, WF>, WF>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
+            grad_cell_f32<CORR, false, PF_CHUNK_GRAD<CORR, WF, DEEP>, WF>(c, sv, fg, fc, cc, phi, phiB, vol, go, g, gcopy, ldc);
     }
     if (tb.lead) {
         const int4 r = ranges_ready(&s_rng);

@@ -456,3 +456,21 @@ def test_fp64_adjoint_forms_equal_the_plain_kernel(cg, gpu, kind, dims, order):
         outs.append(o)
     for a, b in zip(*outs):
         assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+def test_fp64_gradient_forms_on_mixed_cells(cg, gpu):
+    """536 tiles of merged hexahedra take the gradient form with more warps
+    (smaller meshes take the other, tests above): the plain kernel's bits."""
+    import oracle as O
+    import torch
+    mesh = cg.Mesh.from_arrays(O.merge_cells(O.jitter(72, 72, 72, 0.25, seed=5, permute=True), 0.3, 11, max_cells=6),
+                               order=cg.ORDER_MORTON)
+    assert mesh.full_width == 0 and 444 * 256 < mesh.nCells <= 592 * 256
+    phi, phiB = (x.double() for x in _fields(torch, mesh, 41)[:2])
+    off = torch.empty(mesh.nCells + 1, dtype=torch.float64, device="cuda")[1:]
+    off.copy_(phi)
+    out = [torch.full((3, mesh.nCells), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2)]
+    for p, g in zip((phi, off), out):
+        cg.dev_gradient(mesh, cg.PREC_F64, p, phiB, g, stream=torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    assert torch.isfinite(out[0]).all() and torch.equal(*out)
