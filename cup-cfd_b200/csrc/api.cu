@@ -153,6 +153,30 @@ void forms_setup(cupcfd_gpu_mesh *m, int sms) {
     m->gradF64Deep = wf == 0 && places(3) <= places(4);
 }
 
+// Whether an L2-prefetch kernel pays on the mesh. Where the cells are numbered
+// at random (a permuted mesh in owner order: a warp gathers from 31 lines; the
+// other orders and meshes stay below 10), the face records and neighbours that
+// a kernel gathers pass L2's size with the mesh, and then what is fetched ahead
+// only pushes them out. Up to these cells the prefetch pays there, us with /
+// without at 56^3, 88^3, 112^3 and 135^3: FP64 forward 30 / 29, 97 / 95, 265 /
+// 241, 682 / 623; FP32 adjoint 27 / 26, 88 / 88, 202 / 184, 550 / 510; FP32
+// mass adjoint 15 / 15, 43 / 43, 107 / 103, 317 / 292; FP64 corrected gradient
+// (three iterations) 88 / 81, 368 / 354, 1173 / 1068, 2789 / 2565; FP32 75 / 84,
+// 248 / 257, 603 / 592, 1621 / 1559; gradient adjoint FP64 25 / 25, 85 / 86,
+// 196 / 194, 581 / 541, FP32 23 / 27, 76 / 76, 152 / 151, 435 / 410 (144^3);
+// one gradient FP64 15 / 14, 47 / 52, 107 / 113, 233 / 218, FP32 11 / 12, 33 /
+// 33, 66 / 68, 132 / 133 (144^3 177 / 171). The FP64 adjoints gain at all sizes.
+bool prefetch_pays(const cupcfd_gpu_mesh *m, PfKernel k) {
+    if (m->gatherLines < 13.0) return true;
+    switch (k) {
+        case PF_FWD_F64: case PF_ADJ_F32: case PF_CORR_F64: return m->nC <= 1 << 17;
+        case PF_MADJ: case PF_CORR_F32: case PF_GRAD_ADJ_F64: case PF_GRAD_ADJ_F32: return m->nC <= 1 << 20;
+        case PF_GRAD_F64: return m->nC <= 7 << 18;
+        case PF_GRAD_F32: return m->nC <= 10 << 18;
+        default: return true;
+    }
+}
+
 // Builds the per-tile ranges the L2-prefetch kernels of both precisions read
 // and the prefetch distance of each kernel; leaves m->tiles false (plain
 // kernels only) when the faces are not numbered by owner tile (the native
@@ -310,17 +334,18 @@ int launch_grad_once(cupcfd_gpu_mesh *m, int precision, bool corr, bool sgn, con
     unsigned grid = grid_for(m->nC, BLK);
     // the reference's sign on tiled meshes and 16-byte aligned arrays: the
     // L2-prefetch kernels (the same bits)
-    if (m->tiles && !sgn && precision != CUPCFD_PREC_F32REF && aligned16(phi) && aligned16(prev)) {
-#define GRAD_PF(T, G, C, PHI, K, BLOCK, W)                                                                            \
+    const PfKernel pk = precision == CUPCFD_PREC_F64 ? (corr ? PF_CORR_F64 : PF_GRAD_F64) : corr ? PF_CORR_F32 : PF_GRAD_F32;
+    if (m->tiles && !sgn && precision != CUPCFD_PREC_F32REF && aligned16(phi) && aligned16(prev) && prefetch_pays(m, pk)) {
+#define GRAD_PF(T, G, C, PHI, K, BLOCK)                                                                               \
     CG_LAUNCH_PF(m, K, BLOCK, st, m->nC, sell(m), m->G, m->C, m->PHI, (const T *) phi, (const T *) phiB, m->vol,       \
-                 (const T *) prev, (T *) grad, (T *) gcopy, ldc, prefetch_args(m, W))
+                 (const T *) prev, (T *) grad, (T *) gcopy, ldc, prefetch_args(m, pk))
         if (precision == CUPCFD_PREC_F64) {
-            if (corr) GRAD_PF(double, fg64, fc64, cc64, k_corr_f64_pf, PF_BLOCK_GRAD, PF_CORR_F64);
-            else if (m->gradF64Deep) GRAD_PF(double, fg64, fc64, cc64, k_grad_f64_deep_pf, PF_BLOCK_GRAD, PF_GRAD_F64);
-            else GRAD_PF(double, fg64, fc64, cc64, k_grad_f64_pf, PF_BLOCK_GRAD, PF_GRAD_F64);
+            if (corr) GRAD_PF(double, fg64, fc64, cc64, k_corr_f64_pf, PF_BLOCK_GRAD);
+            else if (m->gradF64Deep) GRAD_PF(double, fg64, fc64, cc64, k_grad_f64_deep_pf, PF_BLOCK_GRAD);
+            else GRAD_PF(double, fg64, fc64, cc64, k_grad_f64_pf, PF_BLOCK_GRAD);
         } else {
-            if (corr) GRAD_PF(float, fg32, fc32, cc32, k_corr_f32_pf, PF_BLOCK_GRAD, PF_CORR_F32);
-            else GRAD_PF(float, fg32, fc32, cc32, k_grad_f32_pf, PF_BLOCK_GRAD, PF_GRAD_F32);
+            if (corr) GRAD_PF(float, fg32, fc32, cc32, k_corr_f32_pf, PF_BLOCK_GRAD);
+            else GRAD_PF(float, fg32, fc32, cc32, k_grad_f32_pf, PF_BLOCK_GRAD);
         }
 #undef GRAD_PF
         CG_LAUNCHED();
@@ -481,7 +506,7 @@ extern "C" int cupcfd_gpu_dev_gradient_adjoint(cupcfd_gpu_mesh *m, int32_t preci
     cudaStream_t st = as_stream(stream);
     unsigned grid = grid_for(m->nC, BLK);
     const bool f64 = precision == CUPCFD_PREC_F64, sgn = sign_mode == CUPCFD_SIGN_SIGNED;
-    if (m->tiles && !sgn && aligned16(gbar)) {
+    if (m->tiles && !sgn && aligned16(gbar) && prefetch_pays(m, f64 ? PF_GRAD_ADJ_F64 : PF_GRAD_ADJ_F32)) {
         if (f64)
             CG_LAUNCH_PF(m, k_grad_adj_f64_pf, PF_BLOCK_GRAD_ADJ, st, m->nC, sell(m), m->fg64, m->ivol, (const double *) gbar,
                          (double *) phiBar, (double *) phiBBar, m->nC, prefetch_args(m, PF_GRAD_ADJ_F64));
@@ -510,7 +535,7 @@ extern "C" int cupcfd_gpu_dev_mass_plain_adjoint(cupcfd_gpu_mesh *m, int32_t pre
     if (m->tiles && aligned16(state) && aligned16(mbar) && precision == CUPCFD_PREC_F64)
         CG_LAUNCH_PF(m, k_madj_f64_pf, PF_BLOCK_MADJ_F64, st, m->nC, sell(m), m->fg64, (const double *) state,
                      (const double *) mbar, (double *) stateBar, m->nC, prefetch_args(m, PF_MADJ_F64));
-    else if (m->tiles && aligned16(mbar) && precision == CUPCFD_PREC_F32C)  // the state is 16-byte aligned (check_align)
+    else if (m->tiles && aligned16(mbar) && precision == CUPCFD_PREC_F32C && prefetch_pays(m, PF_MADJ))  // the state is 16-byte aligned (check_align)
         CG_LAUNCH_PF(m, k_madj_f32_pf, PF_BLOCK_MADJ, st, m->nC, sell(m), m->fg32, (const float4 *) state,
                      (const float *) mbar, (float4 *) stateBar, m->nC, prefetch_args(m, PF_MADJ));
     else if (precision == CUPCFD_PREC_F64)
@@ -554,7 +579,7 @@ const char *launch_fwd_f64(const cupcfd_gpu_mesh *m, const void *phi, const void
                            const void *gface, void *grad, void *massFlux, double *part, cudaStream_t st,
                            int *group) {
     *group = 1;
-    if (m->tiles && aligned16(phi) && aligned16(state) && (!gface || aligned16(gface))) {
+    if (m->tiles && aligned16(phi) && aligned16(state) && (!gface || aligned16(gface)) && prefetch_pays(m, PF_FWD_F64)) {
         CG_LAUNCH_PF(m, k_fwd_f64_pf, PF_BLOCK_FWD_F64, st, m->nC, sell(m), m->fg64, (const double *) phi, (const double *) phiB, m->vol,
                            (const double *) state, (const double *) gface, (double *) grad, (double *) massFlux,
                            part, m->nC, prefetch_args(m, PF_FWD_F64));
@@ -642,7 +667,7 @@ extern "C" int cupcfd_gpu_dev_adjoint(cupcfd_gpu_mesh *m, int32_t precision, con
         kt.set_name("k_adj_f64");
         k_adj_f64<<<grid, BLK, 0, st>>>(m->nC, sell(m), m->fg64, (const double *) grad, 2.0, (const double *) state,
                                         (const double *) gface, (double *) phiBar, (double *) phiBBar, (double *) stateBar, m->nC);
-    } else if (m->tiles && aligned16(grad) && aligned16(state) && aligned16(gface)) {
+    } else if (m->tiles && aligned16(grad) && aligned16(state) && aligned16(gface) && prefetch_pays(m, PF_ADJ_F32)) {
         kt.set_name("k_adj_f32_pf");
         CG_LAUNCH_PF(m, k_adj_f32_pf, PF_BLOCK_ADJ, st, m->nC,
                            sell(m), m->fg32, (const float *) grad, 2.f, (const float4 *) state, (const float *) gface,

@@ -474,3 +474,26 @@ def test_fp64_gradient_forms_on_mixed_cells(cg, gpu):
         cg.dev_gradient(mesh, cg.PREC_F64, p, phiB, g, stream=torch.cuda.current_stream())
     torch.cuda.synchronize()
     assert torch.isfinite(out[0]).all() and torch.equal(*out)
+
+
+@pytest.mark.parametrize("order,prefetch", [("ORDER_OWNER", False), ("ORDER_RCM", True)])
+def test_random_numbering_takes_the_plain_kernels(cg, gpu, order, prefetch):
+    """A permuted mesh of over 2^17 cells: kernels that gather more than the
+    L2 prefetch saves run without it where the cells are numbered at random,
+    and with it in an order that keeps neighbours together."""
+    import torch
+    mesh = cg.Mesh.jittered(53, 51, 50, order=getattr(cg, order))
+    assert mesh.nCells > 1 << 17
+    phi, phiB, st, gface = _fields(torch, mesh, 43)
+    _run(cg, torch, mesh, phi, phiB, st, gface, offset=False)
+    assert ("k_adj_f32_pf" in _run.kernels) == prefetch and ("k_adj_f32" in _run.kernels) != prefetch
+    cg.timing_read()
+    cg.timing_enable(True)
+    try:
+        e = lambda *n: torch.zeros(n, dtype=torch.float64, device="cuda")  # noqa: E731
+        cg.dev_forward(mesh, cg.PREC_F64, phi.double(), phiB.double(), st.double().t().contiguous(), e(3, mesh.nCells),
+                       e(mesh.nFaces), gface=gface.double(), loss=e(1), stream=torch.cuda.current_stream())
+        ran = set(cg.timing_read())
+    finally:
+        cg.timing_enable(False)
+    assert ("k_fwd_f64_pf" in ran) == prefetch and ("k_fwd_f64" in ran) != prefetch
