@@ -39,25 +39,32 @@ int scratch(cupcfd_gpu_mesh *m, int slot, size_t n, T **p) {
 
 inline cudaStream_t as_stream(void *s) { return (cudaStream_t) s; }
 
-// The mesh's second and third streams and their events (created on first
-// use): the host forward+adjoint's copy-back and copy-in streams, and the
-// loss reduction beside the gradient adjoint in the device forward+adjoint.
+// The mesh's second stream and its events (created on first use): the loss
+// reduction beside the gradient adjoint in the device forward+adjoint, and the
+// host forward+adjoint's copies back.
 // The stream has the device's highest priority, so that the loss
 // reduction's one block is placed as soon as an SM has room for it, not
 // after the gradient adjoint's blocks.
 #ifndef CUPCFD_AUX_PRIORITY
 #define CUPCFD_AUX_PRIORITY 1
 #endif
-int pipe_init(cupcfd_gpu_mesh *m) {
+int aux_init(cupcfd_gpu_mesh *m) {
     if (m->outStream) return CUPCFD_E_SUCCESS;
     for (cudaEvent_t &e : m->pipeEv)
         if (!e) CG_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    for (cudaEvent_t &e : m->inEv)
-        if (!e) CG_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    if (!m->inStream) CG_CHECK_CUDA(cudaStreamCreateWithFlags(&m->inStream, cudaStreamNonBlocking));
     int lo = 0, hi = 0;
     CG_CHECK_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     CG_CHECK_CUDA(cudaStreamCreateWithPriority(&m->outStream, cudaStreamNonBlocking, CUPCFD_AUX_PRIORITY ? hi : lo));
+    return CUPCFD_E_SUCCESS;
+}
+
+// These and the host forward+adjoint's copy-in stream and events.
+int pipe_init(cupcfd_gpu_mesh *m) {
+    CG_TRY(aux_init(m));
+    if (m->inStream) return CUPCFD_E_SUCCESS;
+    for (cudaEvent_t &e : m->inEv)
+        if (!e) CG_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CG_CHECK_CUDA(cudaStreamCreateWithFlags(&m->inStream, cudaStreamNonBlocking));
     return CUPCFD_E_SUCCESS;
 }
 
@@ -704,7 +711,7 @@ extern "C" int cupcfd_gpu_dev_forward_adjoint(cupcfd_gpu_mesh *m, int32_t precis
         constexpr int WPT = TILE_CELLS / 32;
         double *part;
         CG_TRY(scratch(m, S_LOSS, (size_t) grid * WPT, &part));
-        CG_TRY(pipe_init(m));
+        CG_TRY(aux_init(m));
         PrefetchArgs pf = prefetch_args(m, PF_FWD_MADJ), pfg = prefetch_args(m, PF_GADJ);
         {
             KTIMER("k_fwd_madj_f32_pf", st);
