@@ -62,27 +62,31 @@ def face_counts(n):
     return nC, nFi + nB, nFi, nB
 
 
-def bytes_model(nC, nF, nFi, nB):
+def bytes_model(nC, nF, nFi, nB, rows=True):
     """Algorithmic (compulsory) bytes: each distinct input read once, each
-    output written once; int32 indices; FP64 volumes in both precisions."""
+    output written once; FP64 volumes in both precisions. rows: the cells are
+    numbered along rows (owner order), so that one entry set serves each
+    stretch of lanes: two of six int2 per 32 cells, and a 16-byte head. Else
+    the two cells of a face, int32."""
+    conn = (2 * 48 + 16) * nC // 32 if rows else 4 * nF + 4 * nFi
     return {
         # forward with the mass-flux adjoint (k_fwd_madj_f32_pf): phi 4 + rho,u,v,w 16 + V 8 + grad 12 +
-        # statebar 16 per cell; S 12 + lambda 4 + cell1 4 per face; cell2 4 + g_f 4 + m_f 4 per interior
-        # face; phiB 4 per boundary face
-        "fwd_madj_f32": 56 * nC + 20 * nF + 12 * nFi + 4 * nB,
-        # gradient adjoint (k_gadj_f32_pf): grad 12 + phibar 4 per cell; face geometry and connectivity
-        # as above; phibBar 4 per boundary face
-        "gadj_f32": 16 * nC + 20 * nF + 4 * nFi + 4 * nB,
-        # fused forward, FP32: phi 4 + rho,u,v,w 16 + V 8 + grad 12 per cell;
-        # S 12 + lambda 4 + cell1 4 per face; cell2 4 + m_f 4 per interior face; phiB 4 per boundary face
-        "fwd_f32": 40 * nC + 20 * nF + 8 * nFi + 4 * nB,
-        # adjoint, FP32: grad 12 + state 16 + phibar 4 + statebar 16 per cell; face geometry and
-        # connectivity as above; g_f 4 per interior face; phibBar 4 per boundary face
-        "adj_f32": 48 * nC + 20 * nF + 8 * nFi + 4 * nB,
+        # statebar 16 per cell; S 12 + lambda 4 per face; g_f 4 + m_f 4 per interior face; phiB 4 per
+        # boundary face
+        "fwd_madj_f32": 56 * nC + 16 * nF + 8 * nFi + 4 * nB + conn,
+        # gradient adjoint (k_gadj_f32_pf): grad 12 + phibar 4 per cell; face geometry as above; phibBar 4
+        # per boundary face
+        "gadj_f32": 16 * nC + 16 * nF + 4 * nB + conn,
+        # fused forward, FP32: phi 4 + rho,u,v,w 16 + V 8 + grad 12 per cell; S 12 + lambda 4 per face;
+        # m_f 4 per interior face; phiB 4 per boundary face
+        "fwd_f32": 40 * nC + 16 * nF + 4 * nFi + 4 * nB + conn,
+        # adjoint, FP32: grad 12 + state 16 + phibar 4 + statebar 16 per cell; face geometry as above; g_f 4
+        # per interior face; phibBar 4 per boundary face
+        "adj_f32": 48 * nC + 16 * nF + 4 * nFi + 4 * nB + conn,
         # whole forward+adjoint pipeline: face data and inputs counted once, grad written once and read once
-        "pipeline_f32": 72 * nC + 20 * nF + 12 * nFi + 8 * nB,
+        "pipeline_f32": 72 * nC + 16 * nF + 8 * nFi + 8 * nB + conn,
         # fused forward, FP64: 8-byte reals
-        "fwd_f64": 72 * nC + 32 * nF + 16 * nFi + 8 * nB,
+        "fwd_f64": 72 * nC + 32 * nF + 8 * nFi + 8 * nB + conn,
     }
 
 
@@ -340,8 +344,9 @@ def bench_uvw(cg, mesh, dev, st, g, steps, warmup, peak):
     Inputs drawn as that benchmark draws them (U[1e-6, 1e-2]), gradients
     1e-2 N(0,1). Algorithmic bytes per call: per cell u, v, w, visEff, nine
     gradient components, the cell centre (read) and su..aw (read and written)
-    = 224; per interior face S, lambda, massFlux, two cell ids (read) and
-    rFace (written) = 64; per boundary face its region id = 4."""
+    = 224; per interior face S, lambda, massFlux (read) and rFace (written)
+    = 56; per boundary face its region id = 4; the connectivity as in
+    bytes_model."""
     import torch
     nC, nF, nFi, nB = mesh.nCells, mesh.nFaces, mesh.nInteriorFaces, mesh.nBoundaries
     D = dict(dtype=torch.float64, device=dev)
@@ -369,7 +374,9 @@ def bench_uvw(cg, mesh, dev, st, g, steps, warmup, peak):
     e1.record(st)
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / steps
-    alg = 224 * nC + 64 * nFi + 4 * nB
+    # the two cell ids of a face come from the lists: two runs of 48 bytes and a head per 32 cells along rows
+    rows = mesh.order == cg.ORDER_OWNER
+    alg = 224 * nC + 56 * nFi + 4 * nB + (112 * nC // 32 if rows else 8 * nFi)
     gbs = alg / (ms * 1e-3) / 1e9
     return {"call": "cupcfd_gpu_dev_uvw_face_loop1 (FP64, bit-identical to the reference)", "kernel": "k_uvw_f64_pf",
             "ms_per_call": ms, "value": nF / (ms * 1e-3) / 1e9, "unit": "Gfaces/s", "steps": steps,
@@ -568,7 +575,7 @@ def bench_mesh_files(cg, n=128):
 def workload_config(n, order, world):
     """The `config` of a bench line for the n^3 workload (both arms print it)."""
     nC, nF, nFi, nB = face_counts(n)
-    bm = bytes_model(nC, nF, nFi, nB)
+    bm = bytes_model(nC, nF, nFi, nB, rows=order == 2)
     return {"workload": f"structgen {n}^3 unit cube, FP32-compensated forward+adjoint of "
                         f"GradientPhiGaussDolfyn + FluxMassDolfynFaceLoop",
             "mesh": f"{n}^3", "cells": nC, "faces": nF, "interior_faces": nFi, "boundary_faces": nB,
@@ -818,7 +825,7 @@ def run_gpu(a):
     link = host_link(dev)
 
     # ---- roofline of the dominant kernel, from the device timers of the timed region
-    bm = bytes_model(nC, nF, nFi, nB)
+    bm = bytes_model(nC, nF, nFi, nB, rows=a.order == 2)
     peak, peak_src = measured_peaks()
 
     # ---- the momentum face loop (the next operator after the path), FP64, same mesh
