@@ -1078,10 +1078,11 @@ extern "C" int cupcfd_gpu_flux_mass_dolfyn_face_loop_f32(
 namespace {
 // One part of the benchmark adjoint: the gradient part (phibar, phibBar from
 // g, hscale 2) when state and gface are null, the mass part (stateBar) when g
-// is null and hscale 0. FP32 on tiled meshes with 16-byte aligned arrays: the
-// L2-prefetch kernels of each part (k_gadj_f32_pf, k_madj_f32_pf); else the
-// plain adjoint kernels. Each output's sum is the one the combined kernels
-// form, so the results are theirs.
+// is null and hscale 0. FP32 on tiled meshes of a multiple of four cells: the
+// L2-prefetch kernels of each part (k_gadj_f32_pf, k_madj_f32_pf); else, and in
+// FP64, the plain adjoint kernels (the host link hides most of them: the
+// device calls take the prefetch kernels at any cell count). Each output's sum
+// is the one the combined kernels form, so the results are theirs.
 int launch_adj_part(const cupcfd_gpu_mesh *m, bool f64, const void *g, double hscale, const void *state,
                     const void *gface, void *phiBar, void *phiBBar, void *stateBar, cudaStream_t st) {
     unsigned grid = grid_for(m->nC, BLK);

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(PF_BLOCK_ADJ_F64<WF>, PF_MINB_ADJ_F64<WF, DEEP
 // time; the run form alone 0.555, and roles known at compile time cut its
 // instructions from 752 to about 620 a warp (0.83 against 0.86 ms for the
 // step under the power limit). Five tiles a SM (48 registers) 0.567, three
-// (24 warps) 0.54. It moves 2.07 GB, at 4.3 TB/s; issue slots are 60-70% busy.
+// (24 warps) 0.54. It moves 2.04 GB; issue slots are 61% busy (at 128^3).
 #ifndef CUPCFD_FWD_MADJ_CHUNK
 #define CUPCFD_FWD_MADJ_CHUNK 2
 #endif

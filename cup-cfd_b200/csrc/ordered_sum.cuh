@@ -32,8 +32,9 @@
 // and as many outlet boundaries) a sum takes 4 us to gather and 46 to add
 // (three quarters of it the fifteen or so scans, the rest the additions one
 // by one, 8 cycles each, and the loads), against 215 us for adding one value
-// after another; the solver step's chain of five sums 267 us against 1160.
-// 512 threads with 8 additions each: 1,024 with 4 take 322 us, 256 with 16 323.
+// after another; the solver step's chain of five sums (13 launches) 267 us in
+// short runs, 280 to 290 in calls from Python, against 1160. 512 threads with 8
+// additions each: 1,024 with 4 take 322 us, 256 with 16 323.
 //
 // F32: the chains add in float (the reference's T = float instantiation);
 // values and accumulators stay in double arrays, which hold the float values

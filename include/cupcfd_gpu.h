@@ -262,7 +262,9 @@ int cupcfd_gpu_mesh_check_status(cupcfd_gpu_mesh *mesh, void *stream);
 /* Boundary regions (CupCfdSoAMesh region/boundary arrays): regionType[nRegions]
  * (CUPCFD_RTYPE_*), regionUVW[3*nRegions], regionDen[nRegions] (host, real_size
  * 8) and bndRegion[nBoundaries] (host). Replaces getBoundaryRegionID /
- * getRegionType / getRegionUVW / getRegionDen (UnstructuredMeshInterface.h:1306-1949). */
+ * getRegionType / getRegionUVW / getRegionDen (UnstructuredMeshInterface.h:1306-1949).
+ * A refused call (an unknown type, a region id out of range) leaves the mesh's
+ * regions as they were. */
 int cupcfd_gpu_mesh_set_regions(cupcfd_gpu_mesh *mesh, int32_t nRegions, const int32_t *regionType,
                                 const double *regionUVW, const double *regionDen,
                                 const int32_t *bndRegion, int32_t nBoundaries);
@@ -467,10 +469,11 @@ int cupcfd_gpu_flux_mass_dolfyn_region_loop_f32(cupcfd_gpu_mesh *mesh, float *fl
  * stream: a cudaStream_t (NULL = the legacy default stream).
  * Every array is aligned to its element (the F32C state to 16 bytes);
  * misaligned pointers are rejected with CUPCFD_E_CONFIG_INVALID_VALUE.
- * Forward/adjoint calls whose arrays start on 16-byte boundaries run the
- * L2-prefetch kernels, which ask for each 256-cell tile's contiguous ranges a
- * wave of blocks ahead; other pointers take the plain kernels. Results are
- * bit-identical either way. */
+ * Calls whose arrays start on 16-byte boundaries run the L2-prefetch kernels,
+ * which ask for each 256-cell tile's contiguous ranges a wave of blocks ahead,
+ * where these gain; other pointers, the native numbering and large meshes
+ * numbered at random take the plain kernels. Results are bit-identical either
+ * way. */
 
 /* Reorders n-component cell data (component blocks of nCells, element type
  * src_size / dst_size bytes = 4 or 8, converting) between numberings.
